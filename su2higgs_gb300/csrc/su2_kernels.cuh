@@ -42,6 +42,14 @@ constexpr int NSUMS = 24;
 // ---------------------------------------------------------------------------
 // reductions
 // ---------------------------------------------------------------------------
+// The counters are kept in CTR_COPIES copies of CTR_STRIDE words and summed
+// when they are read: one atomic per warp on one address is a serial chain in
+// L2 (measured 1.1 per ns), which was as long as the pass itself.
+constexpr int CTR_COPIES = 16, CTR_STRIDE = 32;
+constexpr size_t CTR_BYTES = (size_t)CTR_COPIES * CTR_STRIDE * 8;
+__device__ inline unsigned long long* ctr_copy(unsigned long long* ctr, unsigned block) {
+  return ctr + (block & (CTR_COPIES - 1)) * CTR_STRIDE;
+}
 __device__ inline void warp_count(unsigned long long* ctr, int v) {
   // every lane of the warp reaches this call (no early returns in kernels)
   int s = __reduce_add_sync(0xffffffffu, v);
@@ -779,7 +787,7 @@ struct PassArgs {
   void* backup;             // multicanonical backup of the updated field (or null)
   int op;                   // order parameter to reduce (0: none)
   double* partials;         // per-block order-parameter sums (or null)
-  unsigned long long* ctr;  // device counters
+  unsigned long long* ctr;  // device counters (CTR_COPIES copies)
   int* err;                 // device error flag
   // the multicanonical check decided inside the pass (muca_fused_finish):
   // the weight (null: no decision in this launch), arrival counters, the
@@ -812,8 +820,9 @@ __global__ void __launch_bounds__(BS, MINB) k_link(Fields<R> f, PassArgs a) {
     if (a.alg == ALG_HEATBATH) acc = heatbath<R, CC>(f, a.g, cp, c, i, MU, rng, &cap, &err);
     else acc = metro_link<R, CC>(f, a.g, cp, c, i, MU, rng);
   }
-  warp_count(a.ctr + 1, acc);
-  warp_count(a.ctr + 22, cap);
+  unsigned long long* ctr = ctr_copy(a.ctr, blockIdx.x);
+  warp_count(ctr + 1, acc);
+  warp_count(ctr + 22, cap);
   if (err) atomicOr(a.err, 1);
 }
 
@@ -829,7 +838,7 @@ __global__ void __launch_bounds__(BS, MINB) k_u1(Fields<R> f, PassArgs a) {
     SiteRng<R> rng(a.rk, *a.rk.sweep, (uint32_t)i, a.pass);
     acc = metro_u1<R, CC>(f, a.g, cp, c, i, MU, rng);
   }
-  warp_count(a.ctr + 3, acc);
+  warp_count(ctr_copy(a.ctr, blockIdx.x) + 3, acc);
 }
 
 // one parity (or a contiguous block of it) of one doublet / the triplet /
@@ -873,8 +882,9 @@ __global__ void __launch_bounds__(BS, MINB) k_scalar(Fields<R> f, PassArgs a) {
   int base_or = FIELD == 0 ? 10 + a.sub : (FIELD == 1 ? 15 : 19);
   int base_mt = FIELD == 0 ? 6 + a.sub : (FIELD == 1 ? 13 : 17);
   bool any_or = (FIELD == 0 ? cp.alg_d : (FIELD == 1 ? cp.alg_t : cp.alg_s)) == ALG_OR && !a.alg;
-  warp_count(a.ctr + (any_or ? base_or : base_mt), acc);
-  warp_count(a.ctr + 23, fb);
+  unsigned long long* ctr = ctr_copy(a.ctr, blockIdx.x);
+  warp_count(ctr + (any_or ? base_or : base_mt), acc);
+  warp_count(ctr + 23, fb);
   if (a.partials) {
     double s = block_sum(opv);
     if (a.muca) muca_fused_finish(a, s);

@@ -21,7 +21,7 @@ struct __align__(16) ChainDesc {
   CoupT<R> cp;
   uint32_t k0, k1, chain;
   uint32_t* sweep;          // this chain's sweep counter (device word)
-  unsigned long long* ctr;  // this chain's counters [24]
+  unsigned long long* ctr;  // this chain's counters [CTR_COPIES][CTR_STRIDE]
   // multicanonical chains: the weight, the backup of the updated field
   // (indexed like the field), the order parameter's sums over the 32-site
   // warps of a checked half-sweep, the order parameter (0: no weight in
@@ -162,8 +162,9 @@ __device__ __noinline__ void tile_link(const ChainDesc<R>& d, int parity, int al
     if (alg == ALG_HEATBATH) acc = heatbath<R, CC>(d.f, d.g, d.cp, c, i, MU, rng, &cap, &err);
     else acc = metro_link<R, CC>(d.f, d.g, d.cp, c, i, MU, rng);
   }
-  warp_count(d.ctr + 1, acc);
-  warp_count(d.ctr + 22, cap);
+  unsigned long long* ctr = ctr_copy(d.ctr, (unsigned)t0 / BS);
+  warp_count(ctr + 1, acc);
+  warp_count(ctr + 22, cap);
   if (err) atomicOr(errp, 1);
 }
 
@@ -178,7 +179,7 @@ __device__ __noinline__ void tile_u1(const ChainDesc<R>& d, int parity, uint32_t
     SiteRng<R> rng(RngKey{d.k0, d.k1, d.chain, d.sweep}, sweep, (uint32_t)i, pass);
     acc = metro_u1<R, CC>(d.f, d.g, d.cp, c, i, MU, rng);
   }
-  warp_count(d.ctr + 3, acc);
+  warp_count(ctr_copy(d.ctr, (unsigned)t0 / BS) + 3, acc);
 }
 
 // FIELD 0 doublet `sub`, 1 triplet, 2 singlet; force: the pass's forced
@@ -226,8 +227,9 @@ __device__ __noinline__ void tile_scalar(const ChainDesc<R>& d, int parity, int 
   int base_or = FIELD == 0 ? 10 + sub : (FIELD == 1 ? 15 : 19);
   int base_mt = FIELD == 0 ? 6 + sub : (FIELD == 1 ? 13 : 17);
   bool any_or = (FIELD == 0 ? cp.alg_d : (FIELD == 1 ? cp.alg_t : cp.alg_s)) == ALG_OR && !force;
-  warp_count(d.ctr + (any_or ? base_or : base_mt), acc);
-  warp_count(d.ctr + 23, fb);
+  unsigned long long* ctr = ctr_copy(d.ctr, (unsigned)t0 / BS);
+  warp_count(ctr + (any_or ? base_or : base_mt), acc);
+  warp_count(ctr + 23, fb);
 }
 
 template <typename R, int CC, int FIELD, int BS, int MINB>

@@ -99,10 +99,11 @@ struct DevBuf {
   }
 };
 
-// device words of a context: counters, error flag, sweep number, flow
-// marker, and from byte 4096 the arrival counts of a multicanonical check
-// decided inside its update launch (1 + MUCA_MAX_CHUNKS words)
-constexpr size_t CTRBUF_BYTES = 4096 + 4 * (1 + MUCA_MAX_CHUNKS) + 4;
+// device words of a context: error flag, sweep number, flow marker, from byte
+// 4096 the arrival counts of a multicanonical check decided inside its update
+// launch (1 + MUCA_MAX_CHUNKS words), then the counters (CTR_COPIES copies)
+constexpr size_t CTR_OFF = (4096 + 4 * (1 + MUCA_MAX_CHUNKS) + 4 + 255) / 256 * 256;
+constexpr size_t CTRBUF_BYTES = CTR_OFF + CTR_BYTES;
 
 struct su2gpu_ctx {
   su2gpu_params p;
@@ -120,7 +121,7 @@ struct su2gpu_ctx {
   bool borrowed = false;  // fields belong to another allocation (su2gpu_attach)
   Fields<double> f64{};
   Fields<float> f32{};
-  unsigned long long* d_ctr = nullptr;  // [24] counters (accepted + muca)
+  unsigned long long* d_ctr = nullptr;  // counters (accepted + muca), CTR_COPIES copies
   int* d_err = nullptr;
   uint32_t* d_sweep = nullptr;
   unsigned long long* d_fz = nullptr;
@@ -276,7 +277,7 @@ static int create_ctx(const su2gpu_params* p, void* borrowed, const void* copy_f
   }
   if (c->prec == 64) carve(c->f64, (char*)c->fields.p, p, V);
   else carve(c->f32, (char*)c->fields.p, p, V);
-  c->d_ctr = (unsigned long long*)c->ctrbuf.p;
+  c->d_ctr = (unsigned long long*)((char*)c->ctrbuf.p + CTR_OFF);
   c->d_err = (int*)((char*)c->ctrbuf.p + 512);
   c->d_sweep = (uint32_t*)((char*)c->ctrbuf.p + 1024);
   c->d_fz = (unsigned long long*)((char*)c->ctrbuf.p + 1536);
@@ -894,9 +895,9 @@ int su2gpu_autotune(su2gpu_ctx* c, int32_t* choices, float* best_ms) {
   DevBuf tmp, ctr;
   int rc = tmp.ensure(c->fields.n);
   if (rc) return rc;
-  if ((rc = ctr.ensure(4096))) { tmp.release(); return rc; }
+  if ((rc = ctr.ensure(4096 + CTR_BYTES))) { tmp.release(); return rc; }
   CK(cudaMemcpyAsync(tmp.p, c->fields.p, c->fields.n, cudaMemcpyDeviceToDevice, c->st));
-  CK(cudaMemsetAsync(ctr.p, 0, 4096, c->st));
+  CK(cudaMemsetAsync(ctr.p, 0, 4096 + CTR_BYTES, c->st));
   Fields<double> f64;
   Fields<float> f32;
   if (c->prec == 64) carve(f64, (char*)tmp.p, &c->p, c->g.V);
@@ -909,7 +910,7 @@ int su2gpu_autotune(su2gpu_ctx* c, int32_t* choices, float* best_ms) {
   a.cpd = coup_as<double>(c->cp);
   a.cpf = coup_as<float>(c->cp);
   a.rk = RngKey{(uint32_t)c->seed ^ 0x5eedu, (uint32_t)(c->seed >> 32), c->chain, (uint32_t*)((char*)ctr.p + 1024)};
-  a.ctr = (unsigned long long*)ctr.p;
+  a.ctr = (unsigned long long*)((char*)ctr.p + 4096);
   a.err = (int*)((char*)ctr.p + 512);
   a.t_lo = 0;
   a.t_hi = (int)c->g.half;
@@ -981,16 +982,20 @@ int su2gpu_set_variants(su2gpu_ctx* c, const int32_t* choices) {
 
 int su2gpu_get_counters(su2gpu_ctx* c, int64_t* out) {
   if (!c || !out) return SU2GPU_ERR_INVALID;
-  unsigned long long d[SU2GPU_NCOUNTERS];
+  unsigned long long d[CTR_COPIES][CTR_STRIDE];
+  static_assert(SU2GPU_NCOUNTERS <= CTR_STRIDE && sizeof(d) == CTR_BYTES, "counter layout");
   CK(cudaMemcpyAsync(d, c->d_ctr, sizeof(d), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  for (int k = 0; k < SU2GPU_NCOUNTERS; k++) out[k] = (int64_t)d[k] + c->host_tot[k];
+  for (int k = 0; k < SU2GPU_NCOUNTERS; k++) {
+    out[k] = c->host_tot[k];
+    for (int j = 0; j < CTR_COPIES; j++) out[k] += (int64_t)d[j][k];
+  }
   return check_device_error(c);
 }
 
 int su2gpu_reset_counters(su2gpu_ctx* c) {
   if (!c) return SU2GPU_ERR_INVALID;
-  CK(cudaMemsetAsync(c->d_ctr, 0, SU2GPU_NCOUNTERS * 8, c->st));
+  CK(cudaMemsetAsync(c->d_ctr, 0, CTR_BYTES, c->st));
   CK(cudaStreamSynchronize(c->st));
   memset(c->host_tot, 0, sizeof(c->host_tot));
   return SU2GPU_OK;
