@@ -72,7 +72,7 @@ static unsigned l_scalar(int v, int field, const void* f, const PassArgs& a, cud
 }
 static void l_measure(const void* f, const Geom& g, const Coup& cp, const double* alpha, double* partials,
                       unsigned nb, cudaStream_t st) {
-  k_measure<R, CCI><<<nb, BLOCK, 0, st>>>(*(const Fields<R>*)f, g, coup_as<R>(cp), alpha, partials);
+  k_measure<R, CCI><<<nb, meas_threads(g.V), 0, st>>>(*(const Fields<R>*)f, g, coup_as<R>(cp), alpha, partials);
 }
 static void l_flow(const void* fin, const void* fout, const Geom& g, const Coup& cp, double dt,
                    unsigned long long* fz, unsigned nb, cudaStream_t st) {
@@ -143,7 +143,7 @@ void launch_reduce_partials(const double* partials, int np, double* out, cudaStr
 }
 void launch_pool_reduce(const double* partials, int nblocks, const int* first, int base, int nchains, double* out,
                         cudaStream_t st) {
-  if (nchains) k_pool_reduce<<<nchains, 128, 0, st>>>(partials, nblocks, first, base, out);
+  if (nchains) k_pool_reduce<<<nchains, 32 * NSUMS, 0, st>>>(partials, nblocks, first, base, out);
 }
 void launch_pool_next_sweep(uint32_t* const* sweeps, int n, cudaStream_t st, uint32_t inc) {
   if (n) k_pool_next_sweep<<<(n + 255) / 256, 256, 0, st>>>(sweeps, n, inc);

@@ -42,9 +42,11 @@ constexpr int NSUMS = 24;
 // ---------------------------------------------------------------------------
 // reductions
 // ---------------------------------------------------------------------------
-// The counters are kept in CTR_COPIES copies of CTR_STRIDE words and summed
-// when they are read: one atomic per warp on one address is a serial chain in
-// L2 (measured 1.1 per ns), which was as long as the pass itself.
+// A lattice's counters are kept in CTR_COPIES copies of CTR_STRIDE words and
+// summed when they are read: one atomic per warp on one address is a serial
+// chain in L2 (measured 1.1 per ns), as long as a 128^3 lattice's pass itself.
+// The chains of a pool have counters of their own, which spreads the atomics
+// already; copies there only cost their address (384-chain ensemble: 2 %).
 constexpr int CTR_COPIES = 16, CTR_STRIDE = 32;
 constexpr size_t CTR_BYTES = (size_t)CTR_COPIES * CTR_STRIDE * 8;
 __device__ inline unsigned long long* ctr_copy(unsigned long long* ctr, unsigned block) {
@@ -1345,25 +1347,6 @@ __global__ void __launch_bounds__(BLOCK) k_alpha(Fields<R> f, Geom g, CoupT<R> c
   alpha[2 * g.V + t] = (double)alpha_proj(f, g, cp, c, t, 1, 2);
 }
 
-// which of the NSUMS volume sums a content produces
-template <int CC>
-__device__ inline bool sum_active(int k, int rt) {
-  const bool h1 = SU2_HAS(CC, rt, C_H1), h2 = SU2_HAS(CC, rt, C_H2), t = SU2_HAS(CC, rt, C_T),
-             s = SU2_HAS(CC, rt, C_S), u = SU2_HAS(CC, rt, C_U1);
-  const int nh = h2 ? 2 : (h1 ? 1 : 0);
-  switch (k) {
-    case 0: case 1: return true;
-    case 2: return u;
-    case 3: case 4: case 5: return nh > 0;
-    case 6: case 7: case 8: case 9: case 10: return nh > 1;
-    case 11: case 12: case 13: case 15: case 16: return t;
-    case 14: return t && nh > 0;
-    case 17: case 18: case 19: case 20: case 21: return s;
-    case 22: case 23: return s && nh == 1;
-  }
-  return false;
-}
-
 // per-site terms of measure() summed over the block into partials[k][block]
 // Sources of the projected U(1) field strengths alpha_proj (magfield.c:189-216)
 // of the magnetic charge: planes filled by k_alpha (plane 0 = (0,1), 1 = (0,2),
@@ -1599,35 +1582,108 @@ __device__ inline void measure_site(const Fields<R>& f, const Geom& g, const Cou
   m[0] += (double)act;
 }
 
-// sums of m[] over the block (blockDim.x == BLOCK) to partials[k * nblocks + block]
+// Whether the content produces sum k, and the sums a compile-time content
+// produces, numbered: active_sum<CC>(j) is the j-th of nactive_sums<CC>().
+__host__ __device__ constexpr bool sum_active(int k, int content) {
+  const int nh = (content & C_H2) ? 2 : ((content & C_H1) ? 1 : 0);
+  const bool t = content & C_T, s = content & C_S;
+  return k < 2 || (k == 2 && (content & C_U1)) || (k >= 3 && k <= 5 && nh > 0) || (k >= 6 && k <= 10 && nh > 1) ||
+         (k >= 11 && k <= 16 && t && (k != 14 || nh > 0)) || (k >= 17 && k <= 21 && s) || (k >= 22 && s && nh == 1);
+}
 template <int CC>
-__device__ inline void block_sums_out(const double* m, int content, double* partials, int nblocks, int block) {
-  __shared__ double sm[BLOCK / 32][NSUMS];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+constexpr int nactive_sums() {
+  int n = 0;
+  for (int k = 0; k < NSUMS; k++) n += sum_active(k, CC);
+  return n;
+}
+template <int CC>
+constexpr int active_sum(int j) {
+  for (int k = 0; k < NSUMS; k++)
+    if (sum_active(k, CC) && j-- == 0) return k;
+  return -1;
+}
+
+// Sums of N (a power of two <= 32) values over the warp, each lane left with
+// one of them: at every step a lane keeps half of its values, adding the other
+// lane's, and hands the other half over, so N values take about N FP64 adds
+// instead of the 5 N of a tree per value (an FP64 instruction holds the pipe
+// for 16 cycles here).  Lane l ends with value l / (32 / N).
+template <int N, int O>
+__device__ inline double warp_sums(const double (&v)[N]) {
+  if constexpr (N == 1) {
+    double r = v[0];
 #pragma unroll
-  for (int k = 0; k < NSUMS; k++) {
-    if (!sum_active<CC>(k, content)) continue;
-    double v = m[k];
+    for (int o = O; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    return r;
+  } else {
+    const bool up = threadIdx.x & O;
+    double w[N / 2];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sm[w][k] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < NSUMS) {
-    double v = 0.0;
-    if (sum_active<CC>(threadIdx.x, content))
-#pragma unroll
-      for (int ww = 0; ww < BLOCK / 32; ww++) v += sm[ww][threadIdx.x];
-    partials[threadIdx.x * nblocks + block] = v;
+    for (int j = 0; j < N / 2; j++) {
+      const double keep = up ? v[j + N / 2] : v[j], send = up ? v[j] : v[j + N / 2];
+      w[j] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+    }
+    return warp_sums<N / 2, O / 2>(w);
   }
 }
 
-// sites of one measurement block: MEAS_SPT per thread, BLOCK apart
+// sums of m[] over the block (blockDim.x a multiple of 32, at most BLOCK) to
+// partials[k * nblocks + block].  The runtime content sums one value after
+// another, skipping those that its fields do not have.
+template <int CC>
+__device__ inline void block_sums_out(const double* m, int content, double* partials, int nblocks, int block) {
+  constexpr int NA = nactive_sums<CC>();
+  constexpr int N = CC == C_GENERIC ? NSUMS : (NA <= 4 ? 4 : (NA <= 8 ? 8 : (NA <= 16 ? 16 : 32)));
+  __shared__ double sm[BLOCK / 32][N];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int j = -1;  // this thread's sum: its place in sm[w]
+  if constexpr (CC == C_GENERIC) {
+#pragma unroll
+    for (int k = 0; k < NSUMS; k++) {
+      if (!sum_active(k, content)) continue;
+      double v = m[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) sm[w][k] = v;
+    }
+    if (threadIdx.x < NSUMS && sum_active(threadIdx.x, content)) j = threadIdx.x;
+  } else {
+    double v[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q] = q < NA ? m[active_sum<CC>(q < NA ? q : 0)] : 0.0;
+    const double r = warp_sums<N, 16>(v);
+    if (lane % (32 / N) == 0) sm[w][lane / (32 / N)] = r;
+#pragma unroll
+    for (int q = 0; q < NA; q++)
+      if (active_sum<CC>(q) == (int)threadIdx.x) j = q;
+  }
+  __syncthreads();
+  if (threadIdx.x < NSUMS) {
+    double x = 0.0;
+    if (j >= 0)
+      for (int ww = 0; ww < (int)blockDim.x / 32; ww++) x += sm[ww][j];
+    partials[threadIdx.x * nblocks + block] = x;
+  }
+}
+
+// Sites per thread of a measurement of V sites: up to MEAS_SPT, which spreads
+// the block's sum over many sites, but no more than leaves about eight warps per
+// SM (the sum depends on the number, so it is a function of the chain's own
+// volume alone).  With 8 everywhere a 16^3 lattice was 4 blocks.
 constexpr int MEAS_SPT = 8;
-constexpr int MEAS_TILE = BLOCK * MEAS_SPT;
+__host__ __device__ inline int meas_spt(int V) {
+  const int s = V / (32 * 8 * 152);
+  return s < 1 ? 1 : (s > MEAS_SPT ? MEAS_SPT : s);
+}
+// threads per block: one warp where blocks of BLOCK would leave SMs idle
+__host__ __device__ inline int meas_threads(int V) { return V <= 2 * 152 * BLOCK ? 32 : BLOCK; }
+inline unsigned meas_blocks(int V) {
+  const int per = meas_spt(V) * meas_threads(V);
+  return (unsigned)((V + per - 1) / per);
+}
 
 // measure() over the whole lattice; alpha = the k_alpha planes (triplet
-// content) or null.  gridDim.x = ceil(V / MEAS_TILE).
+// content) or null.  meas_blocks(V) blocks of meas_threads(V) threads.
 template <typename R, int CC>
 __global__ void __launch_bounds__(BLOCK) k_measure(Fields<R> f, Geom g, CoupT<R> cp, const double* alpha,
                                                    double* partials) {
@@ -1635,8 +1691,9 @@ __global__ void __launch_bounds__(BLOCK) k_measure(Fields<R> f, Geom g, CoupT<R>
 #pragma unroll
   for (int k = 0; k < NSUMS; k++) m[k] = 0.0;
   const AlphaPlanes ap{alpha, g.V};
-  for (int j = 0; j < MEAS_SPT; j++) {
-    int t = ((int)blockIdx.x * MEAS_SPT + j) * BLOCK + threadIdx.x;
+  const int spt = meas_spt(g.V);
+  for (int j = 0; j < spt; j++) {
+    int t = ((int)blockIdx.x * spt + j) * (int)blockDim.x + threadIdx.x;
     if (t < g.V) measure_site<R, CC>(f, g, cp, t, ap, m);
   }
   block_sums_out<CC>(m, cp.content, partials, gridDim.x, blockIdx.x);

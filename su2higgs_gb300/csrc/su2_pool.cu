@@ -67,9 +67,6 @@ __global__ void k_cold_links4d(D4* p, int64_t n) {
   if (k < n) p[k] = D4{1.0, 0.0, 0.0, 0.0};
 }
 
-// device words of a slot: its sweep counter, then (from byte 256) its counters
-constexpr size_t SLOT_BYTES = 256 + CTR_BYTES;
-
 // doubles per site of one chain's host arrays (links 12, U(1) 3, two doublets
 // 8, triplet 3, singlet 1)
 constexpr int STAGE_REALS = 27;
@@ -107,7 +104,7 @@ struct su2gpu_pool {
   std::vector<std::pair<size_t, size_t>> free_list;  // (offset, length), sorted by offset
   std::vector<Slot> slots;
   int max_slots;
-  Buf slotmem;   // per slot: sweep counter word + counters (SLOT_BYTES)
+  Buf slotmem;   // per slot: sweep counter word + 24 counters
   Buf descs;     // ChainDesc<R>[max_slots]
   Buf tiles[NVARIANTS], mtiles, mfirst, sweepptrs, partials, sums, stage, err;
   // the active chains with a multicanonical weight (their slots), the
@@ -241,8 +238,8 @@ ChainDesc<R> make_desc(su2gpu_pool* P, int s, char* arena_base, char* slot_base)
   d.k0 = (uint32_t)sl.seed;
   d.k1 = (uint32_t)(sl.seed >> 32);
   d.chain = sl.chain;
-  d.sweep = (uint32_t*)(slot_base + (size_t)s * SLOT_BYTES);
-  d.ctr = (unsigned long long*)(slot_base + (size_t)s * SLOT_BYTES + 256);
+  d.sweep = (uint32_t*)(slot_base + (size_t)s * 256);
+  d.ctr = (unsigned long long*)(slot_base + (size_t)s * 256 + 32);
   // the weight only on the pool's own fields: the autotuner's scratch copy
   // sweeps without checks, leaving the chain's multicanonical state alone
   if (sl.mdev && arena_base == (char*)P->arena.p) {
@@ -368,8 +365,8 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
     sp.clear();
     for (int s : P->active) {
       first.push_back((int)mt.size());
-      for (int t0 = 0; t0 < P->slots[s].g.V; t0 += MEAS_TILE) mt.push_back(int2{s, t0});
-      sp.push_back((uint32_t*)(sb + (size_t)s * SLOT_BYTES));
+      for (int t0 = 0; t0 < P->slots[s].g.V; t0 += BLOCK * pool_meas_spt(P->slots[s].g.V)) mt.push_back(int2{s, t0});
+      sp.push_back((uint32_t*)(sb + (size_t)s * 256));
     }
     first.push_back((int)mt.size());
     P->nmtiles = (int)mt.size();
@@ -577,7 +574,7 @@ int su2gpu_pool_create(const su2gpu_params* recipe, int64_t arena_bytes, int32_t
     return fail(SU2GPU_ERR_CUDA, "cudaEventCreate failed");
   }
   size_t dsz = P->prec == 64 ? sizeof(ChainDesc<double>) : sizeof(ChainDesc<float>);
-  if ((rc = P->arena.ensure((size_t)arena_bytes)) || (rc = P->slotmem.ensure((size_t)max_chains * SLOT_BYTES)) ||
+  if ((rc = P->arena.ensure((size_t)arena_bytes)) || (rc = P->slotmem.ensure((size_t)max_chains * 256)) ||
       (rc = P->descs.ensure(dsz * max_chains)) || (rc = P->err.ensure(256)) ||
       (rc = P->qstate.ensure(((size_t)max_chains + 1) * sizeof(unsigned)))) {
     su2gpu_pool_destroy(P);
@@ -665,7 +662,7 @@ int su2gpu_pool_add(su2gpu_pool* P, const su2gpu_params* p, uint64_t seed, uint3
   sl.chain = chain;
   char* base = (char*)P->arena.p + off;
   PCK(cudaMemsetAsync(base, 0, bytes, P->st));
-  PCK(cudaMemsetAsync((char*)P->slotmem.p + (size_t)s * SLOT_BYTES, 0, SLOT_BYTES, P->st));
+  PCK(cudaMemsetAsync((char*)P->slotmem.p + (size_t)s * 256, 0, 256, P->st));
   // cold links (setsu2, init.c:18-28): the three link arrays lead the chain's block
   size_t lbytes = align256((size_t)V * 4 * P->rsize());
   for (int d = 0; d < 3; d++) {
@@ -1013,7 +1010,7 @@ int su2gpu_pool_download_many(su2gpu_pool* P, int32_t n, const int32_t* slots, d
 
 int su2gpu_pool_set_sweep(su2gpu_pool* P, int32_t s, uint32_t sweep) {
   if (!P || s < 0 || s >= P->max_slots || !P->slots[s].active) return fail(SU2GPU_ERR_INVALID, "no such chain slot");
-  PCK(cudaMemcpyAsync((char*)P->slotmem.p + (size_t)s * SLOT_BYTES, &sweep, 4, cudaMemcpyHostToDevice, P->st));
+  PCK(cudaMemcpyAsync((char*)P->slotmem.p + (size_t)s * 256, &sweep, 4, cudaMemcpyHostToDevice, P->st));
   PCK(cudaStreamSynchronize(P->st));
   return SU2GPU_OK;
 }
@@ -1745,13 +1742,10 @@ int su2gpu_pool_enqueue_measure(su2gpu_pool* P, double* device_sums, int32_t max
 
 int su2gpu_pool_counters(su2gpu_pool* P, int32_t s, int64_t* out) {
   if (!P || !out || s < 0 || s >= P->max_slots || !P->slots[s].active) return fail(SU2GPU_ERR_INVALID, "no such chain slot");
-  unsigned long long d[CTR_COPIES][CTR_STRIDE];
-  PCK(cudaMemcpyAsync(d, (char*)P->slotmem.p + (size_t)s * SLOT_BYTES + 256, sizeof(d), cudaMemcpyDeviceToHost, P->st));
+  unsigned long long d[SU2GPU_NCOUNTERS];
+  PCK(cudaMemcpyAsync(d, (char*)P->slotmem.p + (size_t)s * 256 + 32, sizeof(d), cudaMemcpyDeviceToHost, P->st));
   PCK(cudaStreamSynchronize(P->st));
-  for (int k = 0; k < SU2GPU_NCOUNTERS; k++) {
-    out[k] = P->slots[s].tot[k];
-    for (int j = 0; j < CTR_COPIES; j++) out[k] += (int64_t)d[j][k];
-  }
+  for (int k = 0; k < SU2GPU_NCOUNTERS; k++) out[k] = (int64_t)d[k] + P->slots[s].tot[k];
   return SU2GPU_OK;
 }
 

@@ -21,7 +21,7 @@ struct __align__(16) ChainDesc {
   CoupT<R> cp;
   uint32_t k0, k1, chain;
   uint32_t* sweep;          // this chain's sweep counter (device word)
-  unsigned long long* ctr;  // this chain's counters [CTR_COPIES][CTR_STRIDE]
+  unsigned long long* ctr;  // this chain's counters [24]
   // multicanonical chains: the weight, the backup of the updated field
   // (indexed like the field), the order parameter's sums over the 32-site
   // warps of a checked half-sweep, the order parameter (0: no weight in
@@ -162,9 +162,8 @@ __device__ __noinline__ void tile_link(const ChainDesc<R>& d, int parity, int al
     if (alg == ALG_HEATBATH) acc = heatbath<R, CC>(d.f, d.g, d.cp, c, i, MU, rng, &cap, &err);
     else acc = metro_link<R, CC>(d.f, d.g, d.cp, c, i, MU, rng);
   }
-  unsigned long long* ctr = ctr_copy(d.ctr, (unsigned)t0 / BS);
-  warp_count(ctr + 1, acc);
-  warp_count(ctr + 22, cap);
+  warp_count(d.ctr + 1, acc);
+  warp_count(d.ctr + 22, cap);
   if (err) atomicOr(errp, 1);
 }
 
@@ -179,7 +178,7 @@ __device__ __noinline__ void tile_u1(const ChainDesc<R>& d, int parity, uint32_t
     SiteRng<R> rng(RngKey{d.k0, d.k1, d.chain, d.sweep}, sweep, (uint32_t)i, pass);
     acc = metro_u1<R, CC>(d.f, d.g, d.cp, c, i, MU, rng);
   }
-  warp_count(ctr_copy(d.ctr, (unsigned)t0 / BS) + 3, acc);
+  warp_count(d.ctr + 3, acc);
 }
 
 // FIELD 0 doublet `sub`, 1 triplet, 2 singlet; force: the pass's forced
@@ -227,9 +226,8 @@ __device__ __noinline__ void tile_scalar(const ChainDesc<R>& d, int parity, int 
   int base_or = FIELD == 0 ? 10 + sub : (FIELD == 1 ? 15 : 19);
   int base_mt = FIELD == 0 ? 6 + sub : (FIELD == 1 ? 13 : 17);
   bool any_or = (FIELD == 0 ? cp.alg_d : (FIELD == 1 ? cp.alg_t : cp.alg_s)) == ALG_OR && !force;
-  unsigned long long* ctr = ctr_copy(d.ctr, (unsigned)t0 / BS);
-  warp_count(ctr + (any_or ? base_or : base_mt), acc);
-  warp_count(ctr + 23, fb);
+  warp_count(d.ctr + (any_or ? base_or : base_mt), acc);
+  warp_count(d.ctr + 23, fb);
 }
 
 template <typename R, int CC, int FIELD, int BS, int MINB>
@@ -480,8 +478,14 @@ __global__ void k_pool_next_sweep(uint32_t* const* sweeps, int n, uint32_t inc) 
 }
 #endif
 
-// measurement over every chain: tiles of MEAS_TILE sites of each chain
-// (MEAS_SPT per thread); the block sums go to partials[k][block] and are then
+// Sites per thread of a pool chain's measurement: a pool has other chains to
+// fill the SMs, so only small chains are cut finer than MEAS_SPT.
+__host__ __device__ inline int pool_meas_spt(int V) {
+  return V <= 8192 ? 1 : (V <= 32768 ? 2 : MEAS_SPT);
+}
+
+// measurement over every chain: tiles of pool_meas_spt sites per thread of
+// each chain; the block sums go to partials[k][block] and are then
 // reduced per chain.  The magnetic charge's projections are computed where
 // they are needed (no per-chain scratch planes).
 template <typename R, int CC>
@@ -492,7 +496,8 @@ __global__ void __launch_bounds__(BLOCK) k_pool_measure(PoolArgs a, double* part
   double m[NSUMS];
 #pragma unroll
   for (int k = 0; k < NSUMS; k++) m[k] = 0.0;
-  for (int j = 0; j < MEAS_SPT; j++) {
+  const int spt = pool_meas_spt(d.g.V);
+  for (int j = 0; j < spt; j++) {
     int t = tile.y + j * BLOCK + threadIdx.x;
     if (t < d.g.V) measure_site<R, CC>(d.f, d.g, d.cp, t, AlphaOnTheFly{}, m);
   }
@@ -574,24 +579,17 @@ __global__ void __launch_bounds__(256) k_pool_convert(const void* descs, const C
 #ifdef SU2_WITH_GLOBAL
 // per-chain sums: chain k owns blocks [first[k], first[k+1]) - base of the
 // measure tiles (base: the first block of a group of chains); one block per
-// chain, fixed summation order
+// chain, one warp per sum, fixed summation order (a block that took the sums
+// one after another needed 25 us for its 24 trees)
 __global__ void k_pool_reduce(const double* partials, int nblocks, const int* first, int base, double* out) {
-  __shared__ double red[128];
-  int k = blockIdx.x;
-  int b0 = first[k] - base, b1 = first[k + 1] - base;
-  for (int s = 0; s < NSUMS; s++) {
-    const double* row = partials + (size_t)s * nblocks;
-    double v = 0.0;
-    for (int b = b0 + threadIdx.x; b < b1; b += blockDim.x) v += row[b];
-    red[threadIdx.x] = v;
-    __syncthreads();
-    for (int h = blockDim.x >> 1; h > 0; h >>= 1) {
-      if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[(size_t)k * NSUMS + s] = red[0];
-    __syncthreads();
-  }
+  const int k = blockIdx.x, s = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int b0 = first[k] - base, b1 = first[k + 1] - base;
+  const double* row = partials + (size_t)s * nblocks;
+  double v = 0.0;
+  for (int b = b0 + lane; b < b1; b += 32) v += row[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) out[(size_t)k * NSUMS + s] = v;
 }
 
 #endif  // SU2_WITH_GLOBAL

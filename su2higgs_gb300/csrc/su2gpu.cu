@@ -270,7 +270,7 @@ static int create_ctx(const su2gpu_params* p, void* borrowed, const void* copy_f
   }
   if ((!borrowed && (rc = c->fields.ensure(field_bytes(p, V)))) ||
       (rc = c->ctrbuf.ensure(CTRBUF_BYTES)) ||
-      (rc = c->partials.ensure((size_t)(nblk(V, BLOCK) + 2) * NSUMS * 8)) ||
+      (rc = c->partials.ensure((size_t)(std::max(nblk(V, BLOCK), meas_blocks((int)V)) + 2) * NSUMS * 8)) ||
       (rc = c->sums.ensure(NSUMS * 8))) {
     su2gpu_destroy(c);
     return rc;
@@ -1012,7 +1012,7 @@ static int enqueue_measure(su2gpu_ctx* c, const void* F, const Coup& cp, double*
     c->pops->alpha(F, c->g, cp, (double*)c->alpha.p, c->st);
     CKL();
   }
-  unsigned nb = nblk(V, MEAS_TILE);
+  const unsigned nb = meas_blocks((int)V);
   c->ops->measure(F, c->g, cp, (const double*)c->alpha.p, (double*)c->partials.p, nb, c->st);
   CKL();
   launch_reduce_partials((const double*)c->partials.p, (int)nb, out, c->st);
