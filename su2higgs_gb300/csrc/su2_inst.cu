@@ -13,37 +13,54 @@ namespace su2 {
 using R = SU2_R;
 constexpr int CCI = SU2_CC;
 
+// Threads per block of an update launch over n sites.  FP64: a launch of few
+// warps is cut into blocks of one warp (two where the launch decides a
+// multicanonical check, whose sums take 64 threads), so that no SM quarter has
+// more warps than the others: the FP64 pipe (half a lane a cycle and quarter: a
+// warp instruction holds it for 64 cycles, 76 with the three neighbours busy)
+// is the bound; 16^3 doublet half-sweep 14.9 -> 12.6 us.  Past 16 warps an SM
+// whole blocks balance as well.  FP32 warps hide each other's latency and share
+// their SM's L1: blocks of one warp cost 2-5 % there at every size tried
+// (42 x 12 x 30 to 88 x 72 x 14).
+static unsigned launch_threads(int n, int bs, bool check) {
+  if (sizeof(R) == 4 || (n + 31) / 32 > 152 * 16) return (unsigned)bs;
+  return (unsigned)std::min(bs, check ? 64 : 32);
+}
+
 template <int V>
 static unsigned l_link_v(const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
-  unsigned nb = (unsigned)((a.t_hi - a.t_lo + BS - 1) / BS);
+  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS, false);
+  unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
-  if (a.sub == 0) k_link<R, CCI, 0, BS, MB><<<nb, BS, 0, st>>>(F, a);
-  else if (a.sub == 1) k_link<R, CCI, 1, BS, MB><<<nb, BS, 0, st>>>(F, a);
-  else k_link<R, CCI, 2, BS, MB><<<nb, BS, 0, st>>>(F, a);
+  if (a.sub == 0) k_link<R, CCI, 0, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  else if (a.sub == 1) k_link<R, CCI, 1, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  else k_link<R, CCI, 2, BS, MB><<<nb, bs, 0, st>>>(F, a);
   return nb;
 }
 template <int V>
 static unsigned l_u1_v(const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
-  unsigned nb = (unsigned)((a.t_hi - a.t_lo + BS - 1) / BS);
+  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS, false);
+  unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
-  if (a.sub == 0) k_u1<R, CCI, 0, BS, MB><<<nb, BS, 0, st>>>(F, a);
-  else if (a.sub == 1) k_u1<R, CCI, 1, BS, MB><<<nb, BS, 0, st>>>(F, a);
-  else k_u1<R, CCI, 2, BS, MB><<<nb, BS, 0, st>>>(F, a);
+  if (a.sub == 0) k_u1<R, CCI, 0, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  else if (a.sub == 1) k_u1<R, CCI, 1, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  else k_u1<R, CCI, 2, BS, MB><<<nb, bs, 0, st>>>(F, a);
   return nb;
 }
 template <int V>
 static unsigned l_scalar_v(int field, const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
-  unsigned nb = (unsigned)((a.t_hi - a.t_lo + BS - 1) / BS);
+  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS, a.muca != nullptr);
+  unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
-  if (field == 0) k_scalar<R, CCI, 0, BS, MB><<<nb, BS, 0, st>>>(F, a);
-  else if (field == 1) k_scalar<R, CCI, 1, BS, MB><<<nb, BS, 0, st>>>(F, a);
-  else k_scalar<R, CCI, 2, BS, MB><<<nb, BS, 0, st>>>(F, a);
+  if (field == 0) k_scalar<R, CCI, 0, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  else if (field == 1) k_scalar<R, CCI, 1, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  else k_scalar<R, CCI, 2, BS, MB><<<nb, bs, 0, st>>>(F, a);
   return nb;
 }
 static unsigned l_link(int v, const void* f, const PassArgs& a, cudaStream_t st) {
