@@ -321,6 +321,15 @@ template <typename R>
 __device__ inline Q<R> u1phase(R alpha) {
   return Q<R>{mcos(alpha), (R)0, (R)0, -msin(alpha)};
 }
+// x e^{-i alpha sigma_3}, the FP64 form of qmul(x, u1phase(alpha)): one sincos,
+// and no products by the phase's two zero components -- 8 operations instead
+// of 16, each rounded as qmul rounds it.  (The FP32 kernels keep the full
+// product: what the compiler fuses around it decides their bits.)
+__device__ inline Q<double> qphase(const Q<double>& x, double alpha) {
+  double sn, C;
+  sincos(alpha, &sn, &C);
+  return Q<double>{fma(x.a, C, x.d * sn), fma(C, x.b, x.c * sn), fma(C, x.c, -(x.b * sn)), fma(C, x.d, -(x.a * sn))};
+}
 
 template <typename R>
 struct V3 {

@@ -116,7 +116,10 @@ __device__ inline Q<R> link_staple(const Fields<R>& f, const Geom& g, const Coup
     int xp = shifted(g, c, mu, 1);
     for (int h = 0; h < nh; h++) {
       Q<R> nphi = ldro4<R>(php(f, h), xp);
-      if (HAS(C_U1)) nphi = qmul(nphi, u1phase(a1p(f, mu)[i]));
+      if (HAS(C_U1)) {
+        if constexpr (sizeof(R) == 8) nphi = qphase(nphi, a1p(f, mu)[i]);
+        else nphi = qmul(nphi, u1phase(a1p(f, mu)[i]));
+      }
       Q<R> t = qmul(nphi, qdag(ldro4<R>(php(f, h), i)));
       V.a -= (R)0.5 * t.a;
       V.b -= (R)0.5 * t.b;
@@ -151,7 +154,10 @@ __device__ inline R tripletsq(const V3<R>& a) {
 template <typename R, int CC>
 __device__ inline R hop_trace(const CoupT<R>& cp, const Q<R>& p1, const Q<R>& u, const Q<R>& p2, R alpha) {
   Q<R> t = qmul(u, p2);
-  if (HAS(C_U1)) t = qmul(t, u1phase(alpha));
+  if (HAS(C_U1)) {
+    if constexpr (sizeof(R) == 8) t = qphase(t, alpha);
+    else t = qmul(t, u1phase(alpha));
+  }
   return qdot0(qdag(p1), t);
 }
 template <typename R, int CC>
@@ -238,10 +244,16 @@ __device__ inline Q<R> staple_doublet(const Fields<R>& f, const Geom& g, const C
   for (int d = 0; d < 3; d++) {
     int xp = shifted(g, c, d, 1), xm = shifted(g, c, d, -1);
     Q<R> w = qmul(ldro4<R>(lk(f, d), i), ldro4<R>(php(f, h), xp));
-    if (HAS(C_U1)) w = qmul(w, u1phase(a1p(f, d)[i]));
+    if (HAS(C_U1)) {
+      if constexpr (sizeof(R) == 8) w = qphase(w, a1p(f, d)[i]);
+      else w = qmul(w, u1phase(a1p(f, d)[i]));
+    }
     res.a -= w.a; res.b -= w.b; res.c -= w.c; res.d -= w.d;
     w = qmul(qdag(ldro4<R>(lk(f, d), xm)), ldro4<R>(php(f, h), xm));
-    if (HAS(C_U1)) w = qmul(w, qdag(u1phase(a1p(f, d)[xm])));
+    if (HAS(C_U1)) {
+      if constexpr (sizeof(R) == 8) w = qphase(w, -a1p(f, d)[xm]);
+      else w = qmul(w, qdag(u1phase(a1p(f, d)[xm])));
+    }
     res.a -= w.a; res.b -= w.b; res.c -= w.c; res.d -= w.d;
   }
   return res;
@@ -318,17 +330,25 @@ __device__ inline R localact_u1link(const Fields<R>& f, const Geom& g, const Cou
 
 // ---------------------------------------------------------------------------
 // real root of a x^3 + b x^2 + c x + d (polysolve3, overrelax.c:14-34):
-// Cardano's formula followed by Newton steps on the cubic (one in FP64, two
-// in FP32).  The reference evaluates Cardano's formula in long double: the
-// leading coefficient of these cubics is lambda/4 (~5e-4), so the formula
-// cancels, and in double it lands up to ~1e-11 away (relative) from the
-// long-double root.  The cubic itself is well conditioned near its root
-// (the linear coefficient dominates), so a Newton step brings the double
-// result to the root within rounding, matching the reference's long-double
-// value to ~1e-15.
+// Cardano's formula followed by Newton steps on the cubic.  The reference
+// evaluates Cardano's formula in long double: the leading coefficient of
+// these cubics is lambda/4 (~5e-4), so the formula cancels, and in double it
+// lands up to ~1e-11 away (relative) from the long-double root.  The cubic
+// itself is well conditioned near its root (the linear coefficient
+// dominates), so Newton steps bring the result to the root within rounding,
+// matching the reference's long-double value to ~1e-15.
+// FP32: two Newton steps.  FP64: since the Newton steps, not the formula, fix
+// the accuracy, the start comes from the FP32 root, and the steps multiply by
+// an FP32 reciprocal of the slope: the first leaves ~1e-12 of the root's
+// scale, the second rounding.  FP64 Cardano (a square root, a cube root, two
+// divisions, ~95 FP64 instructions, each holding the pipe 16 cycles) stays
+// for the cubics where that start is no good: the last correction has to be
+// below 1e-10 of the root's scale.
 // ---------------------------------------------------------------------------
+__device__ inline double polysolve3_f64(double a, double b, double c, double d, int* fallback);
 template <typename R>
 __device__ inline R polysolve3(R a, R b, R c, R d, int* fallback) {
+  if constexpr (sizeof(R) == 8) return polysolve3_f64(a, b, c, d, fallback);
   R discr = (R)18 * a * b * c * d - (R)4 * b * b * b * d + b * b * c * c - (R)4 * a * c * c * c - (R)27 * a * a * d * d;
   R del1 = (R)2 * b * b * b - (R)9 * a * b * c + (R)27 * a * a * d;
   R x;
@@ -337,7 +357,7 @@ __device__ inline R polysolve3(R a, R b, R c, R d, int* fallback) {
     A = mcbrt(A);
     x = -(b + A + (b * b - (R)3 * a * c) / A) / ((R)3 * a);
 #pragma unroll
-    for (int it = 0; it < (sizeof(R) == 4 ? 2 : 1); it++) {
+    for (int it = 0; it < 2; it++) {
       R fx = ((a * x + b) * x + c) * x + d;
       R dfx = ((R)3 * a * x + (R)2 * b) * x + c;
       x -= fx / dfx;
@@ -348,7 +368,34 @@ __device__ inline R polysolve3(R a, R b, R c, R d, int* fallback) {
   }
   return x;
 }
-
+// one Newton step with the slope's reciprocal in FP32; the correction is returned
+__device__ inline double newton3(double a, double b, double c, double d, double* x) {
+  const double fx = fma(fma(fma(a, *x, b), *x, c), *x, d);
+  const double dfx = fma(fma(3.0 * a, *x, 2.0 * b), *x, c);
+  const double dx = fx * (double)(1.0f / (float)dfx);
+  *x -= dx;
+  return dx;
+}
+__device__ inline double polysolve3_f64(double a, double b, double c, double d, int* fallback) {
+  const double discr = 18.0 * a * b * c * d - 4.0 * b * b * b * d + b * b * c * c - 4.0 * a * c * c * c - 27.0 * a * a * d * d;
+  if (!(discr < 0.0)) {
+    *fallback = 1;
+    return b / a;
+  }
+  int fb = 0;
+  double x = (double)polysolve3<float>((float)a, (float)b, (float)c, (float)d, &fb);
+  newton3(a, b, c, d, &x);
+  const double dx = newton3(a, b, c, d, &x);
+  // an FP32 root of another branch, an overflow or a NaN fails this test
+  if (!(fabs(dx) <= 1e-10 * fabs(x))) {
+    const double del1 = 2.0 * b * b * b - 9.0 * a * b * c + 27.0 * a * a * d;
+    const double A = cbrt(0.5 * (del1 + a * sqrt(-27.0 * discr)));
+    x = -(b + A + (b * b - 3.0 * a * c) / A) / (3.0 * a);
+    const double fx = ((a * x + b) * x + c) * x + d;
+    x -= fx / ((3.0 * a * x + 2.0 * b) * x + c);
+  }
+  return x;
+}
 // ---------------------------------------------------------------------------
 // local updates.  The overrelaxation updates take their random-number source
 // as a template parameter: the sweep kernels pass the site's stream
@@ -377,8 +424,15 @@ __device__ inline int heatbath(const Fields<R>& f, const Geom& g, const CoupT<R>
   }
   Q<R> V = link_staple<R, CC>(f, g, cp, c, i, mu);
   R a = msqrt(qsq(V));
-  V = qscale(V, (R)-1 / a);
-  a *= (R)2;
+  R ia = 0;  // FP64: 1 / (2 |V|), the one division by the staple's length
+  if constexpr (sizeof(R) == 8) {
+    ia = (R)1 / a;
+    V = qscale(V, -ia);
+    ia *= (R)0.5;
+  } else {
+    V = qscale(V, (R)-1 / a);
+    a *= (R)2;
+  }
   R a0, r1, r2, r3, d;
   int loop = 1;
   do {
@@ -388,8 +442,13 @@ __device__ inline int heatbath(const Fields<R>& f, const Geom& g, const CoupT<R>
       u2 = rng.uni();
       u3 = rng.uni();
     }
-    r1 = -mlog((R)1 - u0) / a;
-    r2 = -mlog((R)1 - u1) / a;
+    if constexpr (sizeof(R) == 8) {
+      r1 = -mlog((R)1 - u0) * ia;
+      r2 = -mlog((R)1 - u1) * ia;
+    } else {
+      r1 = -mlog((R)1 - u0) / a;
+      r2 = -mlog((R)1 - u1) / a;
+    }
     r3 = mcos2pi(u2);
     r3 *= r3;
     d = r1 * r3 + r2;
@@ -423,8 +482,8 @@ __device__ inline int heatbath(const Fields<R>& f, const Geom& g, const CoupT<R>
         return 0;
       }
     }
-    d = msqrt(d);
-    nl = Q<R>{a0, r1 * (rad / d), r2 * (rad / d), r3 * (rad / d)};
+    d = rad / msqrt(d);
+    nl = Q<R>{a0, r1 * d, r2 * d, r3 * d};
   } else {
     // FP32 form: the same uniform direction drawn directly (Archimedes:
     // cos(theta) uniform on [-1,1], azimuth uniform), no rejection loop to
@@ -493,10 +552,93 @@ __device__ inline int metro_link(const Fields<R>& f, const Geom& g, const CoupT<
   return 0;
 }
 
+// The FP64 forms of the updates below, which the FP64 pipe bounds (2 lanes a
+// cycle and SM; an OR pass of a 16^3 lattice spent 319 FP64 instructions per
+// site, 16^3 sweep + measurement 325 -> 276 us with these): each update's
+// action difference is formed once from the staple, and divided by once.
+
+// metro_u1link (metropolis.c:48-70): the plaquettes' change from cos A -
+// cos(A + e) = 2 sin(A + e/2) sin(e/2), five trigonometric functions instead
+// of eight, and the hopping terms' from one gather
+template <int CC>
+__device__ inline int metro_u1_f64(const Fields<double>& f, const Geom& g, const CoupT<double>& cp, const int* c,
+                                   int i, int mu, SiteRng<double>& rng) {
+  using R = double;
+  const R old = a1p(f, mu)[i], e = 0.95 * (rng.uni() - 0.5), eh = 0.5 * cp.r_u1 * e;
+  R sum = 0;
+#pragma unroll
+  for (int nu = 0; nu < 3; nu++) {
+    if (nu == mu) continue;
+    // the link enters the plaquette at the site with +, the one below with -
+    sum += sin(fma(cp.r_u1, u1ptrace(f, g, c, i, mu, nu), eh));
+    int cm[3];
+    shift_coords(g, c, nu, -1, cm);
+    sum -= sin(fma(cp.r_u1, u1ptrace(f, g, cm, shifted(g, c, nu, -1), mu, nu), -eh));
+  }
+  R diff = 2.0 * cp.betau1 * sin(eh) * sum;
+  const int xp = shifted(g, c, mu, 1);
+  for (int h = 0; h < NHIGGS; h++) {
+    const Q<R> p = qdag(ld4<R>(php(f, h), i)), t = qmul(ld4<R>(lk(f, mu), i), ld4<R>(php(f, h), xp));
+    diff -= qdot0(p, qphase(t, old + e)) - qdot0(p, qphase(t, old));
+  }
+  if (!metro_accept(diff, rng)) return 0;
+  a1p(f, mu)[i] = old + e;
+  return 1;
+}
+
+// metro_doublet (metropolis.c:77-106): every hopping term is linear in the
+// field, so dS = (p'-p).s + 3 (p'^2-p^2) + V(p') - V(p) with s =
+// staple_doublet -- the neighbours are multiplied once instead of four times
+template <int CC>
+__device__ inline int metro_doublet_f64(const Fields<double>& f, const Geom& g, const CoupT<double>& cp, const int* c,
+                                        int i, int h, SiteRng<double>& rng) {
+  using R = double;
+  const R d0 = rng.uni() - 0.5, d1 = rng.uni() - 0.5, d2 = rng.uni() - 0.5, d3 = rng.uni() - 0.5;
+  const Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, h);
+  const Q<R> old = ld4<R>(php(f, h), i), nw{old.a + d0, old.b + d1, old.c + d2, old.d + d3};
+  const Q<R> e{nw.a - old.a, nw.b - old.b, nw.c - old.c, nw.d - old.d};
+  const R dsq = e.a * (nw.a + old.a) + e.b * (nw.b + old.b) + e.c * (nw.c + old.c) + e.d * (nw.d + old.d);
+  const R v0 = higgspotential<R, CC>(f, cp, i);
+  st4<R>(php(f, h), i, nw);
+  const R diff = (e.a * s.a + e.b * s.b + e.c * s.c + e.d * s.d) + 3.0 * dsq + (higgspotential<R, CC>(f, cp, i) - v0);
+  if (metro_accept(diff, rng)) return 1;
+  st4<R>(php(f, h), i, old);
+  return 0;
+}
+
+// the overrelaxation of a field with N components p in the action p.s + B p^2
+// + C p^4 (overrelax.c:54-236): p is replaced if u accepts the proposal
+template <int N>
+__device__ inline int overrelax_f64(double (&p)[N], const double (&s)[N], double B, double C, double u,
+                                    int* fallback) {
+  double ss = 0, ps = 0, Ysq = 0;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    ss += s[k] * s[k];
+    ps += p[k] * s[k];
+  }
+  const double F = sqrt(ss), iF = 1.0 / F, X = ps * iF;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const double y = p[k] - X * iF * s[k];
+    Ysq += y * y;
+  }
+  const double cc = B + 2.0 * Ysq * C;
+  const double newX = polysolve3<double>(C, C * X, cc + C * X * X, F + cc * X + C * X * X * X, fallback);
+  const double dV = F + 2.0 * B * X + 4.0 * C * (X * X * X + Ysq * X);
+  const double dVn = F + 2.0 * B * newX + 4.0 * C * (newX * newX * newX + Ysq * newX);
+  if (!(fabs(dV) >= u * fabs(dVn))) return 0;
+  const double k0 = (newX + X) * iF;
+#pragma unroll
+  for (int k = 0; k < N; k++) p[k] = k0 * s[k] - p[k];
+  return 1;
+}
+
 // metro_u1link (metropolis.c:48-70)
 template <typename R, int CC>
 __device__ inline int metro_u1(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i, int mu,
                                SiteRng<R>& rng) {
+  if constexpr (sizeof(R) == 8) return metro_u1_f64<CC>(f, g, cp, c, i, mu, rng);
   R old = a1p(f, mu)[i];
   R a0 = localact_u1link<R, CC>(f, g, cp, c, i, mu);
   a1p(f, mu)[i] = old + (R)0.95 * (rng.uni() - (R)0.5);
@@ -510,6 +652,7 @@ __device__ inline int metro_u1(const Fields<R>& f, const Geom& g, const CoupT<R>
 template <typename R, int CC>
 __device__ inline int metro_doublet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                     int h, SiteRng<R>& rng) {
+  if constexpr (sizeof(R) == 8) return metro_doublet_f64<CC>(f, g, cp, c, i, h, rng);
   const R d0 = rng.uni() - (R)0.5, d1 = rng.uni() - (R)0.5, d2 = rng.uni() - (R)0.5, d3 = rng.uni() - (R)0.5;
   Q<R> old = ld4<R>(php(f, h), i);
   R a0 = localact_doublet<R, CC>(f, g, cp, c, i, h);
@@ -530,6 +673,20 @@ template <typename R, int CC, typename RNG>
 __device__ inline int overrelax_doublet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                         RNG& rng, int* fallback) {
   const R u = rng.uni();
+  if constexpr (sizeof(R) == 8) {
+    const Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, 0), p = ld4<R>(php(f, 0), i);
+    R B = 0.5 * cp.msq + 3.0;
+    if (HAS(C_T)) B += 0.5 * cp.a2 * tripletsq(ld3(f, i));
+    if (HAS(C_S)) {
+      const R S = f.sing[i];
+      B += 0.25 * cp.a1s * S + 0.25 * cp.a2s * S * S;
+    }
+    const R sv[4] = {s.a, s.b, s.c, s.d};
+    R pv[4] = {p.a, p.b, p.c, p.d};
+    if (!overrelax_f64<4>(pv, sv, B, 0.25 * cp.lam, u, fallback)) return 0;
+    st4<R>(php(f, 0), i, Q<R>{pv[0], pv[1], pv[2], pv[3]});
+    return 1;
+  }
   Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, 0);
   Q<R> p = ld4<R>(php(f, 0), i);
   R F = msqrt(s.a * s.a + s.b * s.b + s.c * s.c + s.d * s.d);
@@ -596,8 +753,14 @@ __device__ inline int overrelax_higgs2(const Fields<R>& f, const Geom& g, const 
   }
   R F = msqrt(sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2] + sv[3] * sv[3]);
   R X = 0;
+  if constexpr (sizeof(R) == 8) {
+    const R iF = (R)1 / F;
 #pragma unroll
-  for (int k = 0; k < 4; k++) { sv[k] /= F; X += fr[k] * sv[k]; }
+    for (int k = 0; k < 4; k++) { sv[k] *= iF; X += fr[k] * sv[k]; }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) { sv[k] /= F; X += fr[k] * sv[k]; }
+  }
   R Y[4], Ysq = 0;
 #pragma unroll
   for (int k = 0; k < 4; k++) { Y[k] = fr[k] - X * sv[k]; Ysq += Y[k] * Y[k]; }
@@ -647,6 +810,14 @@ template <typename R, int CC, typename RNG>
 __device__ inline int overrelax_triplet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                         RNG& rng, int* fallback) {
   const R u = rng.uni();
+  if constexpr (sizeof(R) == 8) {
+    const V3<R> s = staple_triplet(f, g, c, i), t = ld3(f, i);
+    const R sv[3] = {s.x, s.y, s.z};
+    R tv[3] = {t.x, t.y, t.z};
+    if (!overrelax_f64<3>(tv, sv, 0.5 * cp.msqT + 3.0, 0.25 * cp.b4, u, fallback)) return 0;
+    st3(f, i, V3<R>{tv[0], tv[1], tv[2]});
+    return 1;
+  }
   V3<R> s = staple_triplet(f, g, c, i);
   V3<R> t = ld3(f, i);
   R F = msqrt(s.x * s.x + s.y * s.y + s.z * s.z);
