@@ -8,7 +8,8 @@
 // directions and may have odd sides (6 -> 3), which the EVEN-first
 // checkerboard layout of the update kernels cannot hold; the plain layout
 // holds any side.  Kernels:
-//   k_to_plain       resident fields (FP64 or FP32) -> plain FP64
+//   k_to_plain       resident fields (FP64 or FP32) -> plain FP64, with the
+//                    projector spinors and the photon phases
 //   k_block          smeared fields of the even sites of one plain lattice ->
 //                    the next, coarser plain lattice
 //   k_plane_ops      per plane x_dir = z the sums of |phi|^2/2, Tr Sigma^2 and
@@ -18,6 +19,8 @@
 //   k_correl_combine per distance d the sums over z of products of plane
 //                    totals at z and z + d (periodic), divided by the volume
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "su2_correl.h"
 #include "su2_kernels.cuh"
@@ -55,6 +58,38 @@ __device__ inline V3<double> ptrip(const PlainLat& p, int n) {
   return V3<double>{p.trip[n], p.trip[p.V + n], p.trip[2 * (size_t)p.V + n]};
 }
 
+__device__ inline Spinor<double> pspin(const PlainLat& p, int n) {
+  const double* b = p.spin + n;
+  return Spinor<double>{b[0], b[p.V], b[2 * (size_t)p.V], b[3 * (size_t)p.V]};
+}
+// the triplet of site n with its projector's spinor
+__device__ inline void st_ptrip(const PlainLat& p, int n, const V3<double>& t) {
+  p.trip[n] = t.x;
+  p.trip[p.V + n] = t.y;
+  p.trip[2 * (size_t)p.V + n] = t.z;
+  const Spinor<double> s = proj_spinor(t);
+  double* b = p.spin + n;
+  b[0] = s.r0;
+  b[p.V] = s.i0;
+  b[2 * (size_t)p.V] = s.r1;
+  b[3 * (size_t)p.V] = s.i1;
+}
+// the photon phases of column x
+__device__ inline void st_phase(const PlainLat& p, int x) {
+#pragma unroll
+  for (int tm = 1; tm <= 2; tm++) {
+    double sn, cs;
+    sincospi(2.0 * ((double)(tm * x) / (double)p.L[0]), &sn, &cs);
+    p.phase[4 * x + 2 * (tm - 1)] = cs;
+    p.phase[4 * x + 2 * (tm - 1) + 1] = sn;
+  }
+}
+
+// FP64 kernels over n sites: blocks of one warp while there are few, so that
+// every SM quarter gets some (a warp's FP64 instruction holds its quarter's
+// pipe for 64 cycles)
+static unsigned plain_threads(int n) { return n <= 32 * 608 * 4 ? 32 : BLOCK; }
+
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(BLOCK) k_to_plain(Fields<R> f, Geom g, int has_phi, int has_trip, PlainLat p) {
@@ -71,9 +106,8 @@ __global__ void __launch_bounds__(BLOCK) k_to_plain(Fields<R> f, Geom g, int has
   }
   if (has_trip) {
     V3<R> a = ld3(f, t);
-    p.trip[n] = (double)a.x;
-    p.trip[p.V + n] = (double)a.y;
-    p.trip[2 * (size_t)p.V + n] = (double)a.z;
+    st_ptrip(p, n, V3<double>{(double)a.x, (double)a.y, (double)a.z});
+    if (t < p.L[0]) st_phase(p, t);
   }
   if (has_phi) {
     Q<R> h = ld4<R>(f.phi[0], t);
@@ -138,8 +172,11 @@ __device__ inline V3<double> smear_triplet(const PlainLat& p, const int* bd, con
 // one site of the coarser lattice b: the fields of the site of s at twice its
 // coordinate in the blocked directions, links smeared in the blocked
 // directions (copied in the others), the triplet smeared over the blocked
-// directions; the doublet is not carried (the reference does not smear it)
-__global__ void __launch_bounds__(BLOCK) k_block(PlainLat s, PlainLat b, int bd0, int bd1, int bd2, int has_trip) {
+// directions; the doublet is not carried (the reference does not smear it).
+// blockIdx.y: the link direction, or 3 the triplet -- a coarse lattice has so
+// few sites that the four parts of one, run by different warps, are the
+// parallelism there is (24^3 -> 12^3: 47 us with one thread per site)
+__global__ void __launch_bounds__(BLOCK) k_block(PlainLat s, PlainLat b, int bd0, int bd1, int bd2) {
   int nb = (int)blockIdx.x * blockDim.x + threadIdx.x;
   if (nb >= b.V) return;
   const int bd[3] = {bd0, bd1, bd2};
@@ -148,47 +185,49 @@ __global__ void __launch_bounds__(BLOCK) k_block(PlainLat s, PlainLat b, int bd0
 #pragma unroll
   for (int d = 0; d < 3; d++) cs[d] = bd[d] ? 2 * cb[d] : cb[d];
   const int ns = plain_index(s, cs);
-#pragma unroll
-  for (int d = 0; d < 3; d++) st_plink(b, nb, d, bd[d] ? smear_link(s, bd, cs, d) : plink(s, ns, d));
-  if (has_trip) {
-    V3<double> t = smear_triplet(s, bd, cs);
-    b.trip[nb] = t.x;
-    b.trip[b.V + nb] = t.y;
-    b.trip[2 * (size_t)b.V + nb] = t.z;
+  const int d = blockIdx.y;
+  if (d < 3) {
+    st_plink(b, nb, d, bd[d] ? smear_link(s, bd, cs, d) : plink(s, ns, d));
+  } else {
+    st_ptrip(b, nb, smear_triplet(s, bd, cs));
+    if (nb < b.L[0]) st_phase(b, nb);
   }
 }
 
-// clover_su2 (su2u1.c:207-274): the four plaquettes of the (d1, d2) plane
-// that start at c, summed
-__device__ inline Q<double> clover(const PlainLat& p, const int* c, int d1, int d2) {
+// the vector part of clover_su2 (su2u1.c:207-274), the sum of the four
+// plaquettes of the (d1, d2) plane that start at c:
+//   U1(x) P U2(x)^+ + U2(x) Q U1(x-1) + U1(x-1)^+ R U2(x-2) + U2(x-2)^+ S U1(x)^+
+// with P = U2(x+1) U1(x+2)^+, Q = U1(x+2-1)^+ U2(x-1)^+, R = U2(x-1-2)^+
+// U1(x-1-2), S = U1(x-2) U2(x+1-2).  A product's vector part is minus that of
+// its conjugate, so the last two terms join the first two:
+//   vec[ U1(x) (P U2(x)^+ - S^+ U2(x-2)) + (U2(x) Q - U2(x-2)^+ R^+) U1(x-1) ],
+// eight full products and two vector parts instead of twelve full ones.
+__device__ inline V3<double> clover_vec(const PlainLat& p, const int* c, int d1, int d2) {
   const int n = plain_index(p, c);
   const int x1 = plain_nb(p, c, d1, 1), x2 = plain_nb(p, c, d2, 1), xm1 = plain_nb(p, c, d1, -1),
             xm2 = plain_nb(p, c, d2, -1), x2m1 = plain_nb(p, c, d2, 1, d1, -1),
             xm12 = plain_nb(p, c, d1, -1, d2, -1), x1m2 = plain_nb(p, c, d1, 1, d2, -1);
-  // U_1(x) U_2(x+1) U_1(x+2)^+ U_2(x)^+
-  Q<double> cl = qmul(plink(p, n, d1), qmul(plink(p, x1, d2), qmul(qdag(plink(p, x2, d1)), qdag(plink(p, n, d2)))));
-  // U_2(x) U_1(x+2-1)^+ U_2(x-1)^+ U_1(x-1)
-  cl = qadd(cl, qmul(plink(p, n, d2),
-                     qmul(qdag(plink(p, x2m1, d1)), qmul(qdag(plink(p, xm1, d2)), plink(p, xm1, d1)))));
-  // U_1(x-1)^+ U_2(x-1-2)^+ U_1(x-1-2) U_2(x-2)
-  cl = qadd(cl, qmul(qdag(plink(p, xm1, d1)),
-                     qmul(qdag(plink(p, xm12, d2)), qmul(plink(p, xm12, d1), plink(p, xm2, d2)))));
-  // U_2(x-2)^+ U_1(x-2) U_2(x+1-2) U_1(x)^+
-  cl = qadd(cl, qmul(qdag(plink(p, xm2, d2)),
-                     qmul(plink(p, xm2, d1), qmul(plink(p, x1m2, d2), qdag(plink(p, n, d1))))));
-  return cl;
+  const Q<double> A = plink(p, n, d1), B = plink(p, n, d2), C = plink(p, xm1, d1), D = plink(p, xm2, d2);
+  const Q<double> P = qmul(plink(p, x1, d2), qdag(plink(p, x2, d1)));
+  const Q<double> Sd = qmul(qdag(plink(p, x1m2, d2)), qdag(plink(p, xm2, d1)));
+  Q<double> u = qmul(P, qdag(B)), v = qmul(Sd, D);
+  const Q<double> X{u.a - v.a, u.b - v.b, u.c - v.c, u.d - v.d};
+  const Q<double> q = qmul(qdag(plink(p, x2m1, d1)), qdag(plink(p, xm1, d2)));
+  const Q<double> Rd = qmul(qdag(plink(p, xm12, d1)), plink(p, xm12, d2));
+  u = qmul(B, q);
+  v = qmul(qdag(D), Rd);
+  const Q<double> Y{u.a - v.a, u.b - v.b, u.c - v.c, u.d - v.d};
+  const Q<double> r = qmul(A, X), t = qmul(Y, C);  // the unused real parts are not computed
+  return V3<double>{r.b + t.b, r.c + t.c, r.d + t.d};
 }
 
 // alpha_proj (magfield.c:189-216) on the plain layout, from the spinors of
 // the projectors and the four link overlaps (the same angle as the
 // reference's product of projected link matrices; see alpha_proj)
 __device__ inline double plain_alpha_proj(const PlainLat& p, const int* c, int d1, int d2, double sqrt_beta) {
-  int c1[3] = {c[0], c[1], c[2]}, c2[3] = {c[0], c[1], c[2]};
-  c1[d1] = wrap(c1[d1] + 1, p.L[d1]);
-  c2[d2] = wrap(c2[d2] + 1, p.L[d2]);
-  const int n = plain_index(p, c), n1 = plain_index(p, c1), n2 = plain_index(p, c2), n12 = plain_nb(p, c1, d2, 1);
-  const Spinor<double> sx = proj_spinor(ptrip(p, n)), s1 = proj_spinor(ptrip(p, n1)), s2 = proj_spinor(ptrip(p, n2)),
-                       s12 = proj_spinor(ptrip(p, n12));
+  const int n = plain_index(p, c), n1 = plain_nb(p, c, d1, 1), n2 = plain_nb(p, c, d2, 1),
+            n12 = plain_nb(p, c, d1, 1, d2, 1);
+  const Spinor<double> sx = pspin(p, n), s1 = pspin(p, n1), s2 = pspin(p, n2), s12 = pspin(p, n12);
   double z1r, z1i, z2r, z2i, z3r, z3i, z4r, z4i;
   link_overlap(sx, plink(p, n, d1), s1, z1r, z1i);
   link_overlap(s1, plink(p, n1, d2), s12, z2r, z2i);
@@ -199,25 +238,28 @@ __device__ inline double plain_alpha_proj(const PlainLat& p, const int* c, int d
   return atan2(pi * qr - pr * qi, pr * qr + pi * qi) * sqrt_beta;
 }
 
-// Per plane z (blockIdx.y) and chunk (blockIdx.x) of its sites: q = 0 the sum
-// of |phi|^2/2 (plane_sum(doubletsq), correlation.c:16-33), 1 Tr Sigma^2, then
-// re/im of the photon operators for (transmom, mode) = (1,0), (2,0), (1,1),
-// (2,1): mode 0 the clover field strength projected on Sigma
+// Per plane z (blockIdx.y) and chunk (blockIdx.x) of its sites, one warp: q = 0
+// the sum of |phi|^2/2 (plane_sum(doubletsq), correlation.c:16-33), 1 Tr
+// Sigma^2, then re/im of the photon operators for (transmom, mode) = (1,0),
+// (2,0), (1,1), (2,1): mode 0 the clover field strength projected on Sigma
 // (projected_photon_operator, correlation.c:99-164), mode 1 twice the
 // projected alpha of the plane (photon_projection_full, correlation.c:207-253),
 // times exp(2 pi i p.x) with p = (transmom, 0, 0) when dir != 0 and p = 0 when
 // dir = 0 (photon_correl, correlation.c:270-274, stops its direction loop after
 // the first direction).  Out: part[(z * chunks + chunk) * NCORR_PLANE + q].
-__global__ void __launch_bounds__(CBLOCK) k_plane_ops(PlainLat p, int dir, int has_phi, int has_trip,
-                                                      double sqrt_beta, int chunks, double* part) {
+// Bound by the FP64 pipe (2 lanes a cycle and SM): ~350 FP64 instructions per
+// site, 650 before the spinors, phases and clover terms were shared.  Chunks of
+// one warp fill the last wave; 48^3: 196 us in 336 blocks of four warps.
+__global__ void __launch_bounds__(32) k_plane_ops(PlainLat p, int dir, int has_phi, int has_trip, double sqrt_beta,
+                                                  int chunks, double* part) {
   const int z = blockIdx.y, chunk = blockIdx.x;
   const int d1 = dir == 0 ? 1 : 0, d2 = dir == 2 ? 1 : 2;
   const int area = p.V / p.L[dir];
   const int per = (area + chunks - 1) / chunks, lo = chunk * per, hi = min(area, lo + per);
-  double m[NCORR_PLANE];
+  double m[16];
 #pragma unroll
-  for (int q = 0; q < NCORR_PLANE; q++) m[q] = 0.0;
-  for (int k = lo + (int)threadIdx.x; k < hi; k += CBLOCK) {
+  for (int q = 0; q < 16; q++) m[q] = 0.0;
+  for (int k = lo + (int)threadIdx.x; k < hi; k += 32) {
     int c[3];
     c[dir] = z;
     c[d1] = k % p.L[d1];
@@ -230,106 +272,91 @@ __global__ void __launch_bounds__(CBLOCK) k_plane_ops(PlainLat p, int dir, int h
     if (has_trip) {
       V3<double> a = ptrip(p, n);
       m[1] += 0.5 * (a.x * a.x + a.y * a.y + a.z * a.z);
-      Q<double> cl = clover(p, c, d1, d2);
-      const double tr = a.x * (cl.b / 4.0) + a.y * (cl.c / 4.0) + a.z * (cl.d / 4.0);
+      const V3<double> cl = clover_vec(p, c, d1, d2);
+      const double tr = 0.25 * (a.x * cl.x + a.y * cl.y + a.z * cl.z);
       const double al = 2.0 * plain_alpha_proj(p, c, d1, d2, sqrt_beta);
 #pragma unroll
-      for (int tm = 1; tm <= 2; tm++) {
-        double sn = 0.0, cs = 1.0;
-        if (dir != 0) sincospi(2.0 * ((double)(tm * c[0]) / (double)p.L[0]), &sn, &cs);
-        m[2 + 2 * (tm - 1)] += tr * cs;
-        m[3 + 2 * (tm - 1)] += tr * sn;
-        m[6 + 2 * (tm - 1)] += al * cs;
-        m[7 + 2 * (tm - 1)] += al * sn;
+      for (int tm = 0; tm < 2; tm++) {
+        const double cs = dir != 0 ? p.phase[4 * c[0] + 2 * tm] : 1.0;
+        const double sn = dir != 0 ? p.phase[4 * c[0] + 2 * tm + 1] : 0.0;
+        m[2 + 2 * tm] += tr * cs;
+        m[3 + 2 * tm] += tr * sn;
+        m[6 + 2 * tm] += al * cs;
+        m[7 + 2 * tm] += al * sn;
       }
     }
   }
-  __shared__ double sm[CBLOCK / 32][NCORR_PLANE];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NCORR_PLANE; q++) {
-    double v = m[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sm[w][q] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < NCORR_PLANE) {
-    double v = 0.0;
-    for (int ww = 0; ww < CBLOCK / 32; ww++) v += sm[ww][threadIdx.x];
-    part[((size_t)z * chunks + chunk) * NCORR_PLANE + threadIdx.x] = v;
-  }
+  const double v = warp_sums<16, 16>(m);
+  if (!(threadIdx.x & 1) && threadIdx.x / 2 < NCORR_PLANE)
+    part[((size_t)z * chunks + chunk) * NCORR_PLANE + threadIdx.x / 2] = v;
 }
 
-__global__ void k_plane_totals(const double* part, int Lz, int chunks, double* tot) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= Lz * NCORR_PLANE) return;
-  const int z = t / NCORR_PLANE, q = t % NCORR_PLANE;
+// the plane totals: block z, warp q, fixed order
+__global__ void k_plane_totals(const double* part, int chunks, double* tot) {
+  const int z = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int k = 0; k < chunks; k++) v += part[((size_t)z * chunks + k) * NCORR_PLANE + q];
-  tot[t] = v;
+  for (int k = lane; k < chunks; k += 32) v += part[((size_t)z * chunks + k) * NCORR_PLANE + q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) tot[(size_t)z * NCORR_PLANE + q] = v;
 }
 
-// measure_correlators' values (correlation.c:350-398) at distance d = thread:
+// measure_correlators' values (correlation.c:350-398) at distance d = block:
 // 4 sum_z h(z) h(z+d) / V (higgs_correlator, doubletsq is half the trace),
 // sum_z s(z) s(z+d) / V, and sum_z O(z) O(z+d)^* / V for the four photon
-// operators (cmult, stddefs.h:93-98); out[d][NCORR]
+// operators (cmult, stddefs.h:93-98); out[d][NCORR].  One warp over z, fixed
+// order (one thread per distance took 33 us for its serial loop over 48 planes)
 __global__ void k_correl_combine(const double* tot, int Lz, double vol, int has_phi, int has_trip, double* out) {
-  const int d = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= Lz / 2) return;
-  double hc = 0.0, sc = 0.0, pre[4] = {0, 0, 0, 0}, pim[4] = {0, 0, 0, 0};
-  for (int z = 0; z < Lz; z++) {
-    const int zd = (z + d) % Lz;
+  const int d = (int)blockIdx.x;
+  double s[16];  // 0 Higgs, 1 Sigma^2, 2 + 2k / 3 + 2k photon re / im
+#pragma unroll
+  for (int q = 0; q < 16; q++) s[q] = 0.0;
+  for (int z = threadIdx.x; z < Lz; z += 32) {
+    const int zd = z + d < Lz ? z + d : z + d - Lz;
     const double* a = tot + (size_t)z * NCORR_PLANE;
     const double* b = tot + (size_t)zd * NCORR_PLANE;
-    hc += a[0] * b[0];
-    sc += a[1] * b[1];
+    s[0] += a[0] * b[0];
+    s[1] += a[1] * b[1];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const double ar = a[2 + 2 * k], ai = a[3 + 2 * k], br = b[2 + 2 * k], bi = -b[3 + 2 * k];
-      pre[k] += ar * br - ai * bi;
-      pim[k] += br * ai + ar * bi;
+      s[2 + 2 * k] += ar * br - ai * bi;
+      s[3 + 2 * k] += br * ai + ar * bi;
     }
   }
-  double* r = out + (size_t)d * NCORR;
-  r[0] = has_phi ? 4.0 * hc / vol : 0.0;
-  r[1] = has_trip ? sc / vol : 0.0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    r[2 + 2 * k] = has_trip ? pre[k] / vol : 0.0;
-    r[3 + 2 * k] = has_trip ? pim[k] / vol : 0.0;
-  }
+  const double v = warp_sums<16, 16>(s);
+  const int q = threadIdx.x / 2;
+  if (!(threadIdx.x & 1) && q < NCORR)
+    out[(size_t)d * NCORR + q] = q == 0 ? (has_phi ? 4.0 * v / vol : 0.0) : (has_trip ? v / vol : 0.0);
 }
 
 // ---------------------------------------------------------------------------
 void launch_to_plain(int prec, const void* f, const Geom& g, int has_phi, int has_trip, const PlainLat& p,
                      cudaStream_t st) {
-  if (prec == 64)
-    k_to_plain<double><<<(g.V + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(*(const Fields<double>*)f, g, has_phi, has_trip,
-                                                                    p);
-  else
-    k_to_plain<float><<<(g.V + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(*(const Fields<float>*)f, g, has_phi, has_trip,
-                                                                   p);
+  const unsigned bs = plain_threads(g.V), nb = ((unsigned)g.V + bs - 1) / bs;
+  if (prec == 64) k_to_plain<double><<<nb, bs, 0, st>>>(*(const Fields<double>*)f, g, has_phi, has_trip, p);
+  else k_to_plain<float><<<nb, bs, 0, st>>>(*(const Fields<float>*)f, g, has_phi, has_trip, p);
 }
 
 void launch_block(const PlainLat& s, const PlainLat& b, const int* bd, int has_trip, cudaStream_t st) {
-  k_block<<<(b.V + BLOCK - 1) / BLOCK, BLOCK, 0, st>>>(s, b, bd[0], bd[1], bd[2], has_trip);
+  const unsigned bs = plain_threads(b.V), nb = ((unsigned)b.V + bs - 1) / bs;
+  k_block<<<dim3(nb, has_trip ? 4 : 3), bs, 0, st>>>(s, b, bd[0], bd[1], bd[2]);
 }
 
-int correl_chunks(const PlainLat& p, int dir, int sm_count) {
+// one warp's sites per chunk, more where that would be over 64 warps per SM
+// in all, as there the chunks' sums weigh more than an even last wave
+int correl_chunks(const PlainLat& p, int dir) {
   const int Lz = p.L[dir], area = p.V / Lz;
-  int chunks = (2 * sm_count + Lz - 1) / Lz;  // about two blocks per SM over all planes
-  const int most = (area + CBLOCK - 1) / CBLOCK;
-  if (chunks > most) chunks = most;
-  return chunks < 1 ? 1 : chunks;
+  const int warps = (area + 31) / 32, per = std::max(1, (int)((int64_t)warps * Lz / (152 * 64)));
+  return (warps + per - 1) / per;
 }
 
 void launch_correlators(const PlainLat& p, int dir, int has_phi, int has_trip, double sqrt_beta, int chunks,
                         double* part, double* tot, double* out, cudaStream_t st) {
   const int Lz = p.L[dir];
-  k_plane_ops<<<dim3(chunks, Lz), CBLOCK, 0, st>>>(p, dir, has_phi, has_trip, sqrt_beta, chunks, part);
-  k_plane_totals<<<(Lz * NCORR_PLANE + 127) / 128, 128, 0, st>>>(part, Lz, chunks, tot);
-  k_correl_combine<<<(Lz / 2 + 63) / 64, 64, 0, st>>>(tot, Lz, (double)p.V, has_phi, has_trip, out);
+  k_plane_ops<<<dim3(chunks, Lz), 32, 0, st>>>(p, dir, has_phi, has_trip, sqrt_beta, chunks, part);
+  k_plane_totals<<<Lz, 32 * NCORR_PLANE, 0, st>>>(part, chunks, tot);
+  if (Lz / 2) k_correl_combine<<<Lz / 2, 32, 0, st>>>(tot, Lz, (double)p.V, has_phi, has_trip, out);
 }
 
 }  // namespace su2

@@ -1303,9 +1303,6 @@ static int block_levels_possible(const int* L, const int* bd, int want) {
 // to the host.
 static int correl_run(su2gpu_ctx* c, int dir, const int* bd, int levels, double* out, PlainLat* last) {
   const int has_phi = c->nh > 0, has_trip = c->has_t;
-  int dev = 0, sm = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
   // sides of every level, then the sizes of the buffers
   std::vector<std::array<int, 3>> Ls(1, std::array<int, 3>{c->g.L[0], c->g.L[1], c->g.L[2]});
   for (int k = 1; k <= levels; k++) {
@@ -1315,14 +1312,14 @@ static int correl_run(su2gpu_ctx* c, int dir, const int* bd, int levels, double*
     Ls.push_back(n);
   }
   auto vol = [](const std::array<int, 3>& L) { return (int64_t)L[0] * L[1] * L[2]; };
-  const size_t n0 = plain_doubles(c->g.V, has_phi, has_trip);
-  const size_t n1 = levels > 0 ? plain_doubles(vol(Ls[1]), 0, has_trip) : 0;
+  const size_t n0 = plain_doubles(c->g.V, c->g.L[0], has_phi, has_trip);
+  const size_t n1 = levels > 0 ? plain_doubles(vol(Ls[1]), Ls[1][0], 0, has_trip) : 0;
   size_t npart = 0, ntot = 0, nout = 0;
   const int first = levels > 0 ? 1 : 0;
   for (int k = first; k <= levels; k++) {
     PlainLat q = make_plain(Ls[k].data(), nullptr, 0, 0);
     const int Lz = Ls[k][dir];
-    npart = std::max(npart, (size_t)Lz * correl_chunks(q, dir, sm) * NCORR_PLANE);
+    npart = std::max(npart, (size_t)Lz * correl_chunks(q, dir) * NCORR_PLANE);
     ntot = std::max(ntot, (size_t)Lz * NCORR_PLANE);
     nout += (size_t)(Lz / 2) * NCORR;
   }
@@ -1336,7 +1333,7 @@ static int correl_run(su2gpu_ctx* c, int dir, const int* bd, int levels, double*
   const double sqb = sqrt(c->p.betasu2);
   double* o = dout;
   if (out && levels == 0) {
-    launch_correlators(cur, dir, has_phi, has_trip, sqb, correl_chunks(cur, dir, sm), part, tot, o, c->st);
+    launch_correlators(cur, dir, has_phi, has_trip, sqb, correl_chunks(cur, dir), part, tot, o, c->st);
     CKL();
     o += (size_t)(Ls[0][dir] / 2) * NCORR;
   }
@@ -1346,7 +1343,7 @@ static int correl_run(su2gpu_ctx* c, int dir, const int* bd, int levels, double*
     CKL();
     cur = nxt;
     if (out) {
-      launch_correlators(cur, dir, 0, has_trip, sqb, correl_chunks(cur, dir, sm), part, tot, o, c->st);
+      launch_correlators(cur, dir, 0, has_trip, sqb, correl_chunks(cur, dir), part, tot, o, c->st);
       CKL();
       o += (size_t)(Ls[k][dir] / 2) * NCORR;
     }
