@@ -252,24 +252,25 @@ __device__ inline Q<R> ld4(const V4<R>* p, int i) {
   V4<R> v = p[i];
   return Q<R>{v.x, v.y, v.z, v.w};
 }
-// A load through the read-only data path, for values no thread writes during
-// the launch (a pass's neighbours of the other parity, the fields it does not
-// update); FP32 4-vectors as one 16-byte load, FP64 through the plain path.
-// Units that define SU2_COHERENT_LOADS (the persistent sweep kernel, whose
-// later passes read what its earlier passes wrote) use the plain path, since
-// the read-only path is not coherent with writes made during the launch.
-template <typename R>
-__device__ inline Q<R> ldro4(const V4<R>* p, int i) {
+// A load through the read-only data path (RO), for values no thread writes
+// during the launch; FP32 4-vectors as one 16-byte load, FP64 through the plain
+// path.  Units that define SU2_COHERENT_LOADS take the plain path by default:
+// the read-only path is not coherent with writes made during the launch, and
+// their kernels run while earlier passes are still writing (the persistent and
+// team sweeps, passes that start early).
 #ifdef SU2_COHERENT_LOADS
-  return ld4<R>(p, i);
+constexpr bool RO_DEFAULT = false;
 #else
-  if constexpr (sizeof(R) == 4) {
+constexpr bool RO_DEFAULT = true;
+#endif
+template <typename R, bool RO = RO_DEFAULT>
+__device__ inline Q<R> ldro4(const V4<R>* p, int i) {
+  if constexpr (RO && sizeof(R) == 4) {
     float4 v = __ldg((const float4*)p + i);
     return Q<R>{v.x, v.y, v.z, v.w};
   } else {
     return ld4<R>(p, i);
   }
-#endif
 }
 template <typename R>
 __device__ inline void st4(V4<R>* p, int i, const Q<R>& q) {

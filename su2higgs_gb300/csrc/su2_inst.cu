@@ -2,6 +2,9 @@
 // times with -DSU2_R=<double|float> -DSU2_CC=<content mask or -1>
 // -DSU2_OPS=<table name>; the generic units also carry the content-free
 // kernels (-DSU2_WITH_PREC=<table name>) and, for FP64, the non-template ones.
+// Fields are read with plain loads (SU2_COHERENT_LOADS): the passes start before
+// the pass that wrote their inputs has drained (su2_launch.cuh).
+#define SU2_COHERENT_LOADS 1
 #include <algorithm>
 
 #include "su2_kernels.cuh"
@@ -34,9 +37,9 @@ static unsigned l_link_v(const void* f, const PassArgs& a, cudaStream_t st) {
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
-  if (a.sub == 0) k_link<R, CCI, 0, BS, MB><<<nb, bs, 0, st>>>(F, a);
-  else if (a.sub == 1) k_link<R, CCI, 1, BS, MB><<<nb, bs, 0, st>>>(F, a);
-  else k_link<R, CCI, 2, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  if (a.sub == 0) launch_dependent(k_link<R, CCI, 0, BS, MB>, nb, bs, st, F, a);
+  else if (a.sub == 1) launch_dependent(k_link<R, CCI, 1, BS, MB>, nb, bs, st, F, a);
+  else launch_dependent(k_link<R, CCI, 2, BS, MB>, nb, bs, st, F, a);
   return nb;
 }
 template <int V>
@@ -46,9 +49,9 @@ static unsigned l_u1_v(const void* f, const PassArgs& a, cudaStream_t st) {
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
-  if (a.sub == 0) k_u1<R, CCI, 0, BS, MB><<<nb, bs, 0, st>>>(F, a);
-  else if (a.sub == 1) k_u1<R, CCI, 1, BS, MB><<<nb, bs, 0, st>>>(F, a);
-  else k_u1<R, CCI, 2, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  if (a.sub == 0) launch_dependent(k_u1<R, CCI, 0, BS, MB>, nb, bs, st, F, a);
+  else if (a.sub == 1) launch_dependent(k_u1<R, CCI, 1, BS, MB>, nb, bs, st, F, a);
+  else launch_dependent(k_u1<R, CCI, 2, BS, MB>, nb, bs, st, F, a);
   return nb;
 }
 template <int V>
@@ -58,9 +61,9 @@ static unsigned l_scalar_v(int field, const void* f, const PassArgs& a, cudaStre
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
-  if (field == 0) k_scalar<R, CCI, 0, BS, MB><<<nb, bs, 0, st>>>(F, a);
-  else if (field == 1) k_scalar<R, CCI, 1, BS, MB><<<nb, bs, 0, st>>>(F, a);
-  else k_scalar<R, CCI, 2, BS, MB><<<nb, bs, 0, st>>>(F, a);
+  if (field == 0) launch_dependent(k_scalar<R, CCI, 0, BS, MB>, nb, bs, st, F, a);
+  else if (field == 1) launch_dependent(k_scalar<R, CCI, 1, BS, MB>, nb, bs, st, F, a);
+  else launch_dependent(k_scalar<R, CCI, 2, BS, MB>, nb, bs, st, F, a);
   return nb;
 }
 static unsigned l_link(int v, const void* f, const PassArgs& a, cudaStream_t st) {
@@ -89,7 +92,9 @@ static unsigned l_scalar(int v, int field, const void* f, const PassArgs& a, cud
 }
 static void l_measure(const void* f, const Geom& g, const Coup& cp, const double* alpha, double* partials,
                       unsigned nb, cudaStream_t st) {
-  k_measure<R, CCI><<<nb, meas_threads(g.V), 0, st>>>(*(const Fields<R>*)f, g, coup_as<R>(cp), alpha, partials);
+  const unsigned bs = meas_threads(g.V);
+  launch_dependent(k_measure<R, CCI>, nb, bs, st, *(const Fields<R>*)f, g, coup_as<R>(cp), alpha,
+                   partials);
 }
 static void l_flow(const void* fin, const void* fout, const Geom& g, const Coup& cp, double dt,
                    unsigned long long* fz, unsigned nb, cudaStream_t st) {
@@ -112,11 +117,14 @@ static void p_restore(int field, const void* f, const MucaDev* m, const void* ba
                       cudaStream_t st) {
   if (hi <= lo) return;
   unsigned nb = std::min<unsigned>(nblk(hi - lo, 256), 304);
-  if (field == 0) k_muca_restore<R, 0><<<nb, 256, 0, st>>>(*(const Fields<R>*)f, m, backup, h, lo, hi);
-  else k_muca_restore<R, 1><<<nb, 256, 0, st>>>(*(const Fields<R>*)f, m, backup, h, lo, hi);
+  if (field == 0)
+    launch_dependent(k_muca_restore<R, 0>, nb, 256, st, *(const Fields<R>*)f, m, backup, h, (int)lo, (int)hi);
+  else
+    launch_dependent(k_muca_restore<R, 1>, nb, 256, st, *(const Fields<R>*)f, m, backup, h, (int)lo, (int)hi);
 }
 static void p_alpha(const void* f, const Geom& g, const Coup& cp, double* alpha, cudaStream_t st) {
-  k_alpha<R><<<nblk(g.V, BLOCK), BLOCK, 0, st>>>(*(const Fields<R>*)f, g, coup_as<R>(cp), alpha);
+  const unsigned nb = nblk(g.V, BLOCK);
+  launch_dependent(k_alpha<R>, nb, BLOCK, st, *(const Fields<R>*)f, g, coup_as<R>(cp), alpha);
 }
 static void p_import(const void* f, int64_t V, int kind, int h, const double* src, cudaStream_t st) {
   k_import<R><<<nblk(V * 3, 256), 256, 0, st>>>(*(const Fields<R>*)f, V, kind, h, src);
@@ -156,14 +164,14 @@ void launch_muca_set_param(MucaDev* w, const double* partials, int np, double vo
   k_muca_set_param<<<1, 256, 0, st>>>(w, partials, np, vol, parity);
 }
 void launch_reduce_partials(const double* partials, int np, double* out, cudaStream_t st) {
-  k_reduce_partials<<<NSUMS, 256, 0, st>>>(partials, np, out);
+  launch_dependent(k_reduce_partials, NSUMS, 256, st, partials, np, out);
 }
 void launch_pool_reduce(const double* partials, int nblocks, const int* first, int base, int nchains, double* out,
                         cudaStream_t st) {
   if (nchains) k_pool_reduce<<<nchains, 32 * NSUMS, 0, st>>>(partials, nblocks, first, base, out);
 }
 void launch_pool_next_sweep(uint32_t* const* sweeps, int n, cudaStream_t st, uint32_t inc) {
-  if (n) k_pool_next_sweep<<<(n + 255) / 256, 256, 0, st>>>(sweeps, n, inc);
+  if (n) launch_dependent(k_pool_next_sweep, (n + 255) / 256, 256, st, sweeps, n, inc);
 }
 #endif
 

@@ -11,6 +11,7 @@
 #pragma once
 
 #include "su2_common.cuh"
+#include "su2_launch.cuh"
 
 namespace su2 {
 
@@ -80,7 +81,7 @@ __device__ inline double block_sum(double v) {
 // SU(2) gauge part
 // ---------------------------------------------------------------------------
 // su2staple_wilson (staples.c:84-115)
-template <typename R>
+template <typename R, bool RO = RO_DEFAULT>
 __device__ inline Q<R> wilson_staple(const Fields<R>& f, const Geom& g, const int* c, int i, int mu) {
   Q<R> tot{(R)0, (R)0, (R)0, (R)0};
   int xp = shifted(g, c, mu, 1);
@@ -90,9 +91,9 @@ __device__ inline Q<R> wilson_staple(const Fields<R>& f, const Geom& g, const in
     int xn = shifted(g, c, nu, 1);
     int xpm = shifted(g, c, mu, 1, nu, -1);
     int xm = shifted(g, c, nu, -1);
-    Q<R> up = qmul(qmul(ldro4<R>(lk(f, nu), xp), qdag(ldro4<R>(lk(f, mu), xn))), qdag(ldro4<R>(lk(f, nu), i)));
+    Q<R> up = qmul(qmul(ldro4<R, RO>(lk(f, nu), xp), qdag(ldro4<R, RO>(lk(f, mu), xn))), qdag(ldro4<R, RO>(lk(f, nu), i)));
     tot = qadd(tot, up);
-    Q<R> lo = qmul(qmul(qdag(ldro4<R>(lk(f, nu), xpm)), qdag(ldro4<R>(lk(f, mu), xm))), ldro4<R>(lk(f, nu), xm));
+    Q<R> lo = qmul(qmul(qdag(ldro4<R, RO>(lk(f, nu), xpm)), qdag(ldro4<R, RO>(lk(f, mu), xm))), ldro4<R, RO>(lk(f, nu), xm));
     tot = qadd(tot, lo);
   }
   return tot;
@@ -982,6 +983,7 @@ __device__ inline const CoupT<float>& coup<float>(const PassArgs& a) { return a.
 // neighbour offset and field pointer of the staple is fixed at compile time
 template <typename R, int CC, int MU, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_link(Fields<R> f, PassArgs a) {
+  dependent_wait();
   const CoupT<R>& cp = coup<R>(a);
   int t = a.t_lo + (int)blockIdx.x * blockDim.x + threadIdx.x;
   int acc = 0, cap = 0, err = 0;
@@ -993,6 +995,7 @@ __global__ void __launch_bounds__(BS, MINB) k_link(Fields<R> f, PassArgs a) {
     if (a.alg == ALG_HEATBATH) acc = heatbath<R, CC>(f, a.g, cp, c, i, MU, rng, &cap, &err);
     else acc = metro_link<R, CC>(f, a.g, cp, c, i, MU, rng);
   }
+  dependents_go();
   unsigned long long* ctr = ctr_copy(a.ctr, blockIdx.x);
   warp_count(ctr + 1, acc);
   warp_count(ctr + 22, cap);
@@ -1001,6 +1004,7 @@ __global__ void __launch_bounds__(BS, MINB) k_link(Fields<R> f, PassArgs a) {
 
 template <typename R, int CC, int MU, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_u1(Fields<R> f, PassArgs a) {
+  dependent_wait();
   const CoupT<R>& cp = coup<R>(a);
   int t = a.t_lo + (int)blockIdx.x * blockDim.x + threadIdx.x;
   int acc = 0;
@@ -1011,6 +1015,7 @@ __global__ void __launch_bounds__(BS, MINB) k_u1(Fields<R> f, PassArgs a) {
     SiteRng<R> rng(a.rk, *a.rk.sweep, (uint32_t)i, a.pass);
     acc = metro_u1<R, CC>(f, a.g, cp, c, i, MU, rng);
   }
+  dependents_go();
   warp_count(ctr_copy(a.ctr, blockIdx.x) + 3, acc);
 }
 
@@ -1019,6 +1024,7 @@ __global__ void __launch_bounds__(BS, MINB) k_u1(Fields<R> f, PassArgs a) {
 // sums of the order parameter over the new ones
 template <typename R, int CC, int FIELD, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_scalar(Fields<R> f, PassArgs a) {
+  dependent_wait();
   const CoupT<R>& cp = coup<R>(a);
   int t = a.t_lo + (int)blockIdx.x * blockDim.x + threadIdx.x;
   int acc = 0, fb = 0;
@@ -1055,6 +1061,7 @@ __global__ void __launch_bounds__(BS, MINB) k_scalar(Fields<R> f, PassArgs a) {
   int base_or = FIELD == 0 ? 10 + a.sub : (FIELD == 1 ? 15 : 19);
   int base_mt = FIELD == 0 ? 6 + a.sub : (FIELD == 1 ? 13 : 17);
   bool any_or = (FIELD == 0 ? cp.alg_d : (FIELD == 1 ? cp.alg_t : cp.alg_s)) == ALG_OR && !a.alg;
+  dependents_go();
   unsigned long long* ctr = ctr_copy(a.ctr, blockIdx.x);
   warp_count(ctr + (any_or ? base_or : base_mt), acc);
   warp_count(ctr + 23, fb);
@@ -1081,6 +1088,7 @@ __global__ void __launch_bounds__(BLOCK) k_orderparam(Fields<R> f, Geom g, int p
 // the flag)
 template <typename R, int FIELD>
 __global__ void k_muca_restore(Fields<R> f, const MucaDev* m, const void* backup, int h, int lo, int hi) {
+  dependent_wait();
   if (m->last_accept) return;
   for (int i = lo + (int)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += (int)(gridDim.x * blockDim.x)) {
     if (FIELD == 0) {
@@ -1507,6 +1515,7 @@ __device__ inline R alpha_proj(const Fields<R>& f, const Geom& g, const CoupT<R>
 // alpha(x; 0,1), alpha(x; 0,2), alpha(x; 1,2) for every site
 template <typename R>
 __global__ void __launch_bounds__(BLOCK) k_alpha(Fields<R> f, Geom g, CoupT<R> cp, double* alpha) {
+  dependent_wait();
   int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.V) return;
   int parity = t >= g.half;
@@ -1858,6 +1867,7 @@ inline unsigned meas_blocks(int V) {
 template <typename R, int CC>
 __global__ void __launch_bounds__(BLOCK) k_measure(Fields<R> f, Geom g, CoupT<R> cp, const double* alpha,
                                                    double* partials) {
+  dependent_wait();
   double m[NSUMS];
 #pragma unroll
   for (int k = 0; k < NSUMS; k++) m[k] = 0.0;
@@ -1873,6 +1883,7 @@ __global__ void __launch_bounds__(BLOCK) k_measure(Fields<R> f, Geom g, CoupT<R>
 #ifdef SU2_WITH_GLOBAL
 // fixed-order sum of partials[NSUMS][np] -> out[NSUMS]; one block per sum
 __global__ void k_reduce_partials(const double* partials, int np, double* out) {
+  dependent_wait();
   __shared__ double red[256];
   const double* row = partials + (size_t)blockIdx.x * np;
   double v = 0.0;
@@ -1902,7 +1913,7 @@ __global__ void __launch_bounds__(BLOCK) k_flow(Fields<R> in, Fields<R> out, Geo
 #pragma unroll
   for (int mu = 0; mu < 3; mu++) {
     // grad_force_link (gradflow.c:190-258)
-    Q<R> s = qscale(wilson_staple(in, g, c, i, mu), -cp.beta / (R)8);
+    Q<R> s = qscale(wilson_staple<R, true>(in, g, c, i, mu), -cp.beta / (R)8);  // `in` is not written
     Q<R> U = ld4<R>(lk(in, mu), i);
     if (HAS(C_T)) {
       V3<R> a1 = ld3(in, i), a2 = ld3(in, shifted(g, c, mu, 1));

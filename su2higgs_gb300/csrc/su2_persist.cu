@@ -23,25 +23,25 @@ template <int V>
 static void lp_link_v(const PoolArgs& a, unsigned nb, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
   if (!nb) return;
-  if (a.sub == 0) k_pool_link<R, CCI, 0, BS, MB><<<nb, BS, 0, st>>>(a);
-  else if (a.sub == 1) k_pool_link<R, CCI, 1, BS, MB><<<nb, BS, 0, st>>>(a);
-  else k_pool_link<R, CCI, 2, BS, MB><<<nb, BS, 0, st>>>(a);
+  if (a.sub == 0) launch_dependent(k_pool_link<R, CCI, 0, BS, MB>, nb, BS, st, a);
+  else if (a.sub == 1) launch_dependent(k_pool_link<R, CCI, 1, BS, MB>, nb, BS, st, a);
+  else launch_dependent(k_pool_link<R, CCI, 2, BS, MB>, nb, BS, st, a);
 }
 template <int V>
 static void lp_u1_v(const PoolArgs& a, unsigned nb, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
   if (!nb) return;
-  if (a.sub == 0) k_pool_u1<R, CCI, 0, BS, MB><<<nb, BS, 0, st>>>(a);
-  else if (a.sub == 1) k_pool_u1<R, CCI, 1, BS, MB><<<nb, BS, 0, st>>>(a);
-  else k_pool_u1<R, CCI, 2, BS, MB><<<nb, BS, 0, st>>>(a);
+  if (a.sub == 0) launch_dependent(k_pool_u1<R, CCI, 0, BS, MB>, nb, BS, st, a);
+  else if (a.sub == 1) launch_dependent(k_pool_u1<R, CCI, 1, BS, MB>, nb, BS, st, a);
+  else launch_dependent(k_pool_u1<R, CCI, 2, BS, MB>, nb, BS, st, a);
 }
 template <int V>
 static void lp_scalar_v(int field, const PoolArgs& a, unsigned nb, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
   if (!nb) return;
-  if (field == 0) k_pool_scalar<R, CCI, 0, BS, MB><<<nb, BS, 0, st>>>(a);
-  else if (field == 1) k_pool_scalar<R, CCI, 1, BS, MB><<<nb, BS, 0, st>>>(a);
-  else k_pool_scalar<R, CCI, 2, BS, MB><<<nb, BS, 0, st>>>(a);
+  if (field == 0) launch_dependent(k_pool_scalar<R, CCI, 0, BS, MB>, nb, BS, st, a);
+  else if (field == 1) launch_dependent(k_pool_scalar<R, CCI, 1, BS, MB>, nb, BS, st, a);
+  else launch_dependent(k_pool_scalar<R, CCI, 2, BS, MB>, nb, BS, st, a);
 }
 static void lp_link(int v, const PoolArgs& a, unsigned nb, cudaStream_t st) {
   switch (v) {
@@ -68,10 +68,11 @@ static void lp_scalar(int v, int field, const PoolArgs& a, unsigned nb, cudaStre
   }
 }
 static void lp_restore(const PoolArgs& a, const int* mslots, int n, int kb, cudaStream_t st) {
-  if (n > 0) k_pool_restore<R, PBS, PMB><<<(unsigned)(n * kb), PBS, 0, st>>>(a, mslots, kb);
+  if (n > 0)
+    launch_dependent(k_pool_restore<R, PBS, PMB>, (unsigned)(n * kb), PBS, st, a, mslots, kb);
 }
 static void lp_decide(const PoolArgs& a, const int* mslots, int n, cudaStream_t st) {
-  if (n > 0) k_pool_decide<R, PBS, PMB><<<(unsigned)n, PBS, 0, st>>>(a, mslots);
+  if (n > 0) launch_dependent(k_pool_decide<R, PBS, PMB>, (unsigned)n, PBS, st, a, mslots);
 }
 static void persist_launch(int shape, bool muca, const void* args, unsigned grid, cudaStream_t st) {
   if (!grid) return;

@@ -243,25 +243,34 @@ __device__ __noinline__ void tile_scalar_any(const ChainDesc<R>& d, int parity, 
 template <typename R, int CC, int MU, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_pool_link(PoolArgs a) {
   int2 tile = a.tiles[blockIdx.x];
-  if (bad_tile(a, tile)) return;
-  const ChainDesc<R>& d = stage_desc<R>(a, tile.x);
+  const bool bad = bad_tile(a, tile);
+  const ChainDesc<R>& d = stage_desc<R>(a, bad ? 0 : tile.x);
+  dependent_wait();  // the tables and descriptors are the host's: read before it
+  if (bad) return;
   tile_link<R, CC, MU, BS, MINB>(d, a.parity, a.alg, a.pass, *d.sweep, tile.y, a.err);
+  dependents_go();
 }
 
 template <typename R, int CC, int MU, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_pool_u1(PoolArgs a) {
   int2 tile = a.tiles[blockIdx.x];
-  if (bad_tile(a, tile)) return;
-  const ChainDesc<R>& d = stage_desc<R>(a, tile.x);
+  const bool bad = bad_tile(a, tile);
+  const ChainDesc<R>& d = stage_desc<R>(a, bad ? 0 : tile.x);
+  dependent_wait();  // the tables and descriptors are the host's: read before it
+  if (bad) return;
   tile_u1<R, CC, MU, BS, MINB>(d, a.parity, a.pass, *d.sweep, tile.y);
+  dependents_go();
 }
 
 template <typename R, int CC, int FIELD, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_pool_scalar(PoolArgs a) {
   int2 tile = a.tiles[blockIdx.x];
-  if (bad_tile(a, tile)) return;
-  const ChainDesc<R>& d = stage_desc<R>(a, tile.x);
+  const bool bad = bad_tile(a, tile);
+  const ChainDesc<R>& d = stage_desc<R>(a, bad ? 0 : tile.x);
+  dependent_wait();  // the tables and descriptors are the host's: read before it
+  if (bad) return;
   tile_scalar_any<R, CC, FIELD, BS, MINB>(d, a.parity, a.sub, a.alg, a.pass, *d.sweep, tile.y);
+  dependents_go();
 }
 
 // The decide and restore passes with one launch per pass, over the pool's
@@ -272,11 +281,13 @@ __global__ void __launch_bounds__(BS, MINB) k_pool_scalar(PoolArgs a) {
 template <typename R, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_pool_decide(PoolArgs a, const int* mslots) {
   const int slot = mslots[blockIdx.x];
-  if ((unsigned)slot >= (unsigned)a.nslots) {
+  const bool bad = (unsigned)slot >= (unsigned)a.nslots;
+  const ChainDesc<R>& d = stage_desc<R>(a, bad ? 0 : slot);
+  dependent_wait();
+  if (bad) {
     if (threadIdx.x == 0) atomicOr(a.err, 2);
     return;
   }
-  const ChainDesc<R>& d = stage_desc<R>(a, slot);
   tile_decide<R, BS>(d, a.alg, a.sub, a.parity, a.pass, *d.sweep, 0);
 }
 
@@ -284,6 +295,7 @@ template <typename R, int BS, int MINB>
 __global__ void __launch_bounds__(BS, MINB) k_pool_restore(PoolArgs a, const int* mslots, int kb) {
   const int c = blockIdx.x / kb, b = blockIdx.x - c * kb;
   const int slot = mslots[c];
+  dependent_wait();
   if ((unsigned)slot >= (unsigned)a.nslots) {
     if (threadIdx.x == 0 && b == 0) atomicOr(a.err, 2);
     return;
@@ -473,6 +485,7 @@ __global__ void __launch_bounds__(BS, MINB) k_pool_persist(PersistArgs a) {
 #ifdef SU2_WITH_GLOBAL
 // every active chain's sweep counter + inc
 __global__ void k_pool_next_sweep(uint32_t* const* sweeps, int n, uint32_t inc) {
+  dependent_wait();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) *sweeps[k] += inc;
 }

@@ -56,7 +56,10 @@ void su2gpu_record_error(const char* msg) { set_err("%s", msg); }
 static unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 __global__ void k_set_u32(uint32_t* p, uint32_t v) { *p = v; }
-__global__ void k_inc_u32(uint32_t* p) { *p += 1u; }
+__global__ void k_inc_u32(uint32_t* p) {
+  dependent_wait();
+  *p += 1u;
+}
 __global__ void k_fill_u64(unsigned long long* p, unsigned long long v) { *p = v; }
 
 // layout tables (layout.c:657-756 serial order) from the closed form
@@ -701,7 +704,7 @@ static int enqueue_sweeps(su2gpu_ctx* c, uint32_t first_sweep, int32_t nsweeps, 
       c->st = c->own_st;
       CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
       int rc = enqueue_sweep(c, tot, first_sweep);
-      k_inc_u32<<<1, 1, 0, c->st>>>(c->d_sweep);
+      launch_dependent(k_inc_u32, 1, 1, c->st, c->d_sweep);
       cudaError_t e = cudaStreamEndCapture(c->st, &graph);
       c->st = exec;
       if (rc) return rc;
@@ -720,7 +723,7 @@ static int enqueue_sweeps(su2gpu_ctx* c, uint32_t first_sweep, int32_t nsweeps, 
     for (int s = 0; s < nsweeps; s++) {
       int rc = enqueue_sweep(c, c->host_tot, first_sweep + (uint32_t)s);
       if (rc) return rc;
-      k_inc_u32<<<1, 1, 0, c->st>>>(c->d_sweep);
+      launch_dependent(k_inc_u32, 1, 1, c->st, c->d_sweep);
       CKL();
     }
   }
