@@ -103,6 +103,10 @@ struct PoolOps {
   // the multicanonical decide and restore passes over the chains mslots[0..n)
   void (*pool_restore)(const PoolArgs& a, const int* mslots, int n, int kb, cudaStream_t st);
   void (*pool_decide)(const PoolArgs& a, const int* mslots, int n, cudaStream_t st);
+  // the team sweep of nchains chains (`args`, a TeamArgs): clusters of `blocks`
+  // blocks of `threads`; and the clusters of that shape resident at once
+  cudaError_t (*team)(bool muca, int blocks, int threads, int nchains, const void* args, cudaStream_t st);
+  int (*team_clusters)(bool muca, int blocks, int threads);
 };
 extern const PoolOps persist_f64_generic, persist_f64_fund, persist_f64_adj, persist_f64_su2u1s;
 extern const PoolOps persist_f32_generic, persist_f32_fund, persist_f32_adj, persist_f32_su2u1s;

@@ -100,7 +100,47 @@ static int persist_blocks_per_sm(int shape) {
   return e0 == cudaSuccess && e1 == cudaSuccess ? (n0 < n1 ? n0 : n1) : 0;
 }
 
+static cudaError_t team_config(bool muca, int blocks, int threads, int nchains, cudaStream_t st,
+                               cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+  const void* k = muca ? (const void*)k_pool_team<R, CCI, PBS, PMB, true>
+                       : (const void*)k_pool_team<R, CCI, PBS, PMB, false>;
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = (unsigned)(nchains * blocks);
+  cfg->blockDim = (unsigned)threads;
+  cfg->stream = st;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)blocks;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+  // clusters of 16 blocks are beyond the portable size
+  return cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+static cudaError_t team_launch(bool muca, int blocks, int threads, int nchains, const void* args, cudaStream_t st) {
+  if (nchains <= 0) return cudaSuccess;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  const cudaError_t e = team_config(muca, blocks, threads, nchains, st, &cfg, &at);
+  if (e != cudaSuccess) return e;
+  const TeamArgs& a = *(const TeamArgs*)args;
+  return muca ? cudaLaunchKernelEx(&cfg, k_pool_team<R, CCI, PBS, PMB, true>, a)
+              : cudaLaunchKernelEx(&cfg, k_pool_team<R, CCI, PBS, PMB, false>, a);
+}
+static int team_clusters(bool muca, int blocks, int threads) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  int n = 0;
+  if (team_config(muca, blocks, threads, 1, nullptr, &cfg, &at) != cudaSuccess) return 0;
+  const cudaError_t e = muca ? cudaOccupancyMaxActiveClusters(&n, k_pool_team<R, CCI, PBS, PMB, true>, &cfg)
+                             : cudaOccupancyMaxActiveClusters(&n, k_pool_team<R, CCI, PBS, PMB, false>, &cfg);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 const PoolOps SU2_PERSIST = {PBS, persist_launch, persist_blocks_per_sm, lp_link, lp_u1, lp_scalar, lp_restore,
-                               lp_decide};
+                               lp_decide, team_launch, team_clusters};
 
 }  // namespace su2

@@ -136,6 +136,13 @@ struct su2gpu_pool {
   int seg_tiles = 8, seg_env = 0, seg_tuned = 0;  // seg_tuned: the autotuner's pick (0: none)
   int npasses = 0;  // passes per sweep of the recipe (set at the rebuild)
   int nmuca = 0;    // active chains with a multicanonical weight (set at the rebuild)
+  // the team sweep (k_pool_team) for pools of small chains: whether it is in
+  // effect for the current membership, and its launches -- chains of one team
+  // shape, a range of the slot list each
+  struct Team { int blocks, threads, first, count; };
+  bool team = false;
+  std::vector<Team> teams;
+  Buf teamslots;
   Buf segs;
   std::vector<int4> h_segs;  // (slot, t0, the chain's segment count, 0)
   std::vector<int> h_sfirst;
@@ -187,6 +194,7 @@ static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* o
 static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass);
 static std::vector<int> make_groups(const su2gpu_pool* P, int G, bool light_ends);
 static int sweep_streams(su2gpu_pool* P, int NS, std::vector<cudaStream_t>& ss);
+static int ensure_events(std::vector<cudaEvent_t>& v, size_t n);
 }
 
 namespace {
@@ -259,6 +267,61 @@ void append_segments(const su2gpu_pool* P, int s, int seg, std::vector<int4>& ou
   const int step = kVariantBS[0] * seg;
   const int half = (int)P->slots[s].g.half, nseg = (half + step - 1) / step;
   for (int t0 = 0; t0 < half; t0 += step) out.push_back(int4{s, t0, nseg, 0});
+}
+
+// The team sweep is the automatic choice where every chain fits a team and all
+// teams are resident at once: then each pass of each chain takes its own
+// latency, ~2 us, where a launch per pass takes 4-6 us whatever it covers.  A
+// chain's team: four warps a block (in FP64, one per SM quarter) up to 16
+// blocks, then more threads a block.  FP32 teams end at 16 warps a block (8192
+// sites of a parity, 25^3): beyond, a block's passes take as long as a launch
+// over all SMs.  FP64 warps on one quarter run one after another, so FP64
+// teams end at four warps a block.
+struct TeamShape { int blocks, threads; };
+bool team_shape(int prec, int half, TeamShape* t) {
+  const int w = (half + 31) / 32;  // warps of a pass
+  if (w <= 16) *t = TeamShape{4, 128};
+  else if (w <= 64) *t = TeamShape{TEAM_BLOCKS, 128};
+  else if (prec == 32 && w <= 128) *t = TeamShape{TEAM_BLOCKS, 256};
+  else if (prec == 32 && w <= 256) *t = TeamShape{TEAM_BLOCKS, TEAM_MAX_THREADS};
+  else return false;
+  return true;
+}
+int choose_teams(su2gpu_pool* P, bool fits) {
+  P->team = false;
+  P->teams.clear();
+  if (!fits || P->persist_mode >= 0 || P->grouped || P->persistent || P->active.empty()) return SU2GPU_OK;
+  std::vector<std::pair<int, int>> order;  // (shape, slot)
+  for (int s : P->active) {
+    TeamShape t;
+    if (!team_shape(P->prec, P->slots[s].g.half, &t)) return SU2GPU_OK;
+    order.push_back({t.blocks * 1024 + t.threads, s});
+  }
+  std::stable_sort(order.begin(), order.end(), [](auto& a, auto& b) { return a.first > b.first; });
+  std::vector<int> slots;
+  std::vector<su2gpu_pool::Team> teams;
+  for (auto& o : order) {
+    const int blocks = o.first / 1024, threads = o.first % 1024;
+    if (teams.empty() || teams.back().blocks != blocks || teams.back().threads != threads)
+      teams.push_back({blocks, threads, (int)slots.size(), 0});
+    teams.back().count++;
+    slots.push_back(o.second);
+  }
+  // the shares of the device that the launches fill have to add up to less
+  // than one (placing clusters of several shapes leaves some room unused)
+  double share = 0.0;
+  for (auto& t : teams) {
+    const int n = P->pers->team_clusters(P->nmuca > 0, t.blocks, t.threads);
+    if (n <= 0) return SU2GPU_OK;
+    share += (double)t.count / n;
+  }
+  if (share > 0.9) return SU2GPU_OK;
+  if (int rc = P->teamslots.ensure(slots.size() * sizeof(int))) return rc;
+  PCK(cudaMemcpyAsync(P->teamslots.p, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, P->st));
+  PCK(cudaStreamSynchronize(P->st));  // the list is this function's
+  P->teams.swap(teams);
+  P->team = true;
+  return SU2GPU_OK;
 }
 
 // descriptors and tile tables for the current membership
@@ -346,6 +409,7 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
     } else {
       P->h_groups.clear();
     }
+    if (int rc = choose_teams(P, fits)) return rc;
     P->h_segs.clear();
     P->h_sfirst.clear();
     for (int s : P->active) {
@@ -521,6 +585,43 @@ int enqueue_persist(su2gpu_pool* P, const int4* tiles, int nt, uint32_t* const* 
   return SU2GPU_OK;
 }
 
+// `nsweeps` sweeps of every chain by the teams: one launch per team shape, side
+// by side on the update streams when there are several, then the chains' sweep
+// counters + nsweeps (with sweeps)
+int enqueue_teams(su2gpu_pool* P, uint32_t* const* sweeps, int nchains, int nsweeps, int64_t* tot,
+                  const void* descs = nullptr) {
+  std::vector<PassDesc> passes;
+  sweep_recipe(P->recipe, passes, tot, P->mucamask);
+  TeamArgs A;
+  memset(&A, 0, sizeof(A));
+  A.descs = descs ? descs : P->descs.p;
+  A.npasses = (int)passes.size();
+  A.nsweeps = nsweeps;
+  A.err = (int*)P->err.p;
+  for (size_t k = 0; k < passes.size(); k++) A.passes[k] = passes[k];
+  const int n = (int)P->teams.size();
+  std::vector<cudaStream_t> ss(1, P->st);
+  if (n > 1) {
+    int rc;
+    if ((rc = sweep_streams(P, n, ss)) || (rc = ensure_events(P->grp_ev, (size_t)n + 1))) return rc;
+    PCK(cudaEventRecord(P->grp_ev[0], P->st));
+    for (cudaStream_t st : ss) PCK(cudaStreamWaitEvent(st, P->grp_ev[0], 0));
+  }
+  for (int k = 0; k < n; k++) {
+    const su2gpu_pool::Team& t = P->teams[k];
+    A.slots = (const int*)P->teamslots.p + t.first;
+    PCK(P->pers->team(P->nmuca > 0, t.blocks, t.threads, t.count, &A, ss[k]));
+  }
+  if (n > 1)
+    for (int k = 0; k < n; k++) {
+      PCK(cudaEventRecord(P->grp_ev[k + 1], ss[k]));
+      PCK(cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0));
+    }
+  if (sweeps) launch_pool_next_sweep(sweeps, nchains, P->st, (uint32_t)nsweeps);
+  PCK(cudaGetLastError());
+  return SU2GPU_OK;
+}
+
 bool same_recipe(const su2gpu_params* a, const su2gpu_params* b) {
   return a->content == b->content && a->precision == b->precision && a->algorithm_su2link == b->algorithm_su2link &&
          a->algorithm_u1link == b->algorithm_u1link && a->algorithm_su2doublet == b->algorithm_su2doublet &&
@@ -612,7 +713,7 @@ int su2gpu_pool_destroy(su2gpu_pool* P) {
   P->segs.release();
   P->arena.release(); P->slotmem.release(); P->descs.release(); P->mtiles.release(); P->mfirst.release();
   P->sweepptrs.release(); P->partials.release(); P->sums.release(); P->stage.release(); P->err.release();
-  P->mslots.release();
+  P->mslots.release(); P->teamslots.release();
   for (int v = 0; v < NVARIANTS; v++) P->tiles[v].release();
   for (int k = 0; k < 2; k++)
     if (P->stage_ev[k]) cudaEventDestroy(P->stage_ev[k]);
@@ -1056,6 +1157,8 @@ static int pool_enqueue(su2gpu_pool* P, int32_t nsweeps, int32_t use_graph) {
                                      tot))) {
       return rc;
     }
+  } else if (P->team) {
+    if ((rc = enqueue_teams(P, sweeps, na, nsweeps, tot))) return rc;
   } else if (P->grouped) {
     // the groups' sweeps on grp_NS streams in turn, forked from and joined
     // back into the pool's stream
@@ -1617,6 +1720,10 @@ int su2gpu_pool_launches_per_sweep(su2gpu_pool* P, int32_t* n) {
     *n = 2;
     return SU2GPU_OK;
   }
+  if (P->team) {
+    *n = (int)P->teams.size() + 1;
+    return SU2GPU_OK;
+  }
   const int ngroups = P->grouped ? (int)P->h_groups.size() - 1 : 1;
   // the recipe's passes per sweep, in the order of enqueue_pool_sweep
   const su2gpu_params& p = P->recipe;
@@ -1971,7 +2078,21 @@ int su2gpu_pool_autotune(su2gpu_pool* P, int32_t* choices, float* best_ms) {
     }
   } else if (!rc && P->persist_mode == -1 && P->nmuca == 0 && P->active.size() >= 8) {
     const int na = (int)P->active.size();
-    if (base_ms <= 0.f && (rc = time_grouped(P, desc2.p, 1, 1, reps, &base_ms))) {
+    if (P->team) {
+      float ms = 0.f;
+      for (int r = -1; r < reps && !rc; r++) {
+        int64_t t1[SU2GPU_NCOUNTERS] = {0};
+        cudaEventRecord(e0, P->st);
+        if ((rc = enqueue_teams(P, nullptr, na, TUNE_SWEEPS, t1, desc2.p))) break;
+        cudaEventRecord(e1, P->st);
+        PCK(cudaEventSynchronize(e1));
+        float t = 0.f;
+        cudaEventElapsedTime(&t, e0, e1);
+        if (r >= 0) ms += t;
+      }
+      if (!rc) base_ms = ms / reps / TUNE_SWEEPS;
+    }
+    if (!rc && base_ms <= 0.f && (rc = time_grouped(P, desc2.p, 1, 1, reps, &base_ms))) {
       // base_ms stays unset; rc is returned below
     }
     // (groups, streams): on the 384-chain ensemble (11 M sites) groups of

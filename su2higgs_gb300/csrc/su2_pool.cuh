@@ -355,6 +355,18 @@ struct PersistArgs {
   PassDesc passes[PERSIST_MAX_PASSES];
 };
 
+// the team sweep (k_pool_team below)
+constexpr int TEAM_BLOCKS = 16;       // blocks of the largest cluster
+constexpr int TEAM_MAX_THREADS = 512;
+
+struct TeamArgs {
+  const void* descs;  // ChainDesc<R>[...]
+  const int* slots;   // the chains of this launch, one per cluster
+  int npasses, nsweeps;
+  int* err;
+  PassDesc passes[PERSIST_MAX_PASSES];
+};
+
 #ifdef SU2_COHERENT_LOADS
 __device__ inline unsigned ld_acquire_gpu(const unsigned* p) {
   unsigned v;
@@ -479,6 +491,40 @@ __global__ void __launch_bounds__(BS, MINB) k_pool_persist(PersistArgs a) {
       atomicAdd(a.done + tile.x, 1u);
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// The team sweep, for pools of small chains: a chain belongs to one cluster of
+// blocks, which runs all its passes of all the sweeps in one launch with a
+// cluster barrier after each pass.  A pass of a small chain is a few warps'
+// work, about 1.5 us of load and arithmetic latency; launched by itself it
+// takes 4-6 us (start, tile table, descriptor, drain), which no number of
+// chains hides below ~6000 warps a pass.  Here a block stages its chain's
+// descriptor once.  Block r of C takes the sites r NT, r NT + C NT, ... (NT
+// threads) of every pass.  The barrier's release and acquire order a pass's
+// writes before the next pass's reads across the cluster; chains never touch
+// one another.
+// ---------------------------------------------------------------------------
+__device__ inline void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename R, int CC, int BS, int MINB, bool MUCA>
+__global__ void __launch_bounds__(TEAM_MAX_THREADS, BS * MINB / TEAM_MAX_THREADS) k_pool_team(TeamArgs a) {
+  unsigned rank, C;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+  const ChainDesc<R>& d = stage_desc_slot<R>(a.descs, a.slots[blockIdx.x / C]);
+  const uint32_t sweep0 = *d.sweep;
+  const int half = d.g.half, step = (int)(C * blockDim.x);
+  for (int s = 0; s < a.nsweeps; s++)
+    for (int k = 0; k < a.npasses; k++) {
+      const PassDesc p = a.passes[k];
+      for (int t0 = (int)(rank * blockDim.x); t0 < half; t0 += step)
+        persist_tile<R, CC, BS, MINB, MUCA>(d, p, sweep0 + (uint32_t)s, t0, a.err);
+      cluster_barrier();
+    }
 }
 #endif  // SU2_COHERENT_LOADS
 
