@@ -111,6 +111,7 @@ struct su2gpu_pool {
   // restore launch's blocks per chain, and the half-sweeps that any of them
   // checks (bit 0 / 1: doublet 0 / 1, bit 2: triplet)
   Buf mslots;
+  std::vector<int> h_mfirst;  // chains with a weight before each active chain (+ the end)
   int restore_kb = 1, mucamask = 0;
   int64_t stage_sites = 0;          // sites each staging half holds (STAGE_REALS doubles per site)
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
@@ -176,6 +177,7 @@ struct su2gpu_pool {
   int grp_G = 0, grp_NS = 1;
   std::vector<int> h_groups;
   bool grouped = false;
+  int run_NS = 1;  // the streams in effect: grp_NS, or the automatic choice's
   std::vector<cudaEvent_t> cyc_ev;
   // n: sweeps per replay; per_pass: one launch per pass even where the group
   // would sweep persistently
@@ -324,6 +326,36 @@ int choose_teams(su2gpu_pool* P, bool fits) {
   return SU2GPU_OK;
 }
 
+// The groups of the automatic choice, for pools that neither the persistent nor
+// the team sweep takes: GROUP_STREAMS groups at a time on as many streams.
+// Passes of different groups then fill each other's launch gaps, ramps and
+// tails (one launch per pass issues instructions half of the time, four streams
+// three quarters), and where the pool exceeds L2, the chains in flight stay in
+// it from pass to pass: as many rounds as keep them to GROUP_BYTES, or one
+// round up to ONE_ROUND_BYTES.  Measured, us for the sweeps of a pool, one
+// launch per pass against this choice (the best of 50 group and stream counts):
+// 96 chains of 157 MB 7247 / 5148 (5148), 48 of 79 MB 3073 / 2638 (2608), 64 of
+// 39 MB 1709 / 1307 (1306), 20 of 28 MB 1452 / 1084 (1069); of 157 MB in one
+// round 6583, in rounds of 105 MB 6019.  FP64 pools, bound by the FP64 pipe, gain
+// the gaps alone (10 chains 1289 / 1044), so only pools of one round are grouped.
+constexpr int GROUP_STREAMS = 4;
+constexpr int64_t GROUP_BYTES = 60 << 20, ONE_ROUND_BYTES = 90 << 20;
+void choose_groups(su2gpu_pool* P) {
+  if (P->grouped || P->persistent || P->team || P->persist_mode >= 0 || P->active.size() < 2) return;
+  int64_t bytes = 0;
+  for (int s : P->active) bytes += (int64_t)P->slots[s].bytes;
+  if (P->prec == 64 && bytes > ONE_ROUND_BYTES) return;
+  const int rounds = bytes <= ONE_ROUND_BYTES ? 1 : (int)((bytes + GROUP_BYTES - 1) / GROUP_BYTES);
+  P->h_groups = make_groups(P, rounds * GROUP_STREAMS, false);
+  const int G = (int)P->h_groups.size() - 1;
+  if (G < 2) {  // one chain dominates
+    P->h_groups.clear();
+    return;
+  }
+  P->grouped = true;
+  P->run_NS = std::min(G, GROUP_STREAMS);
+}
+
 // descriptors and tile tables for the current membership
 int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullptr, void* descs = nullptr) {
   char* ab = (char*)(arena_base ? arena_base : P->arena.p);
@@ -380,7 +412,9 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
     std::vector<int> ms;
     int64_t mhalf = 1;
     P->mucamask = 0;
-    for (int s : P->active)
+    P->h_mfirst.clear();
+    for (int s : P->active) {
+      P->h_mfirst.push_back((int)ms.size());
       if (P->slots[s].mdev && P->slots[s].mop) {
         const int op = P->slots[s].mop;
         ms.push_back(s);
@@ -388,7 +422,9 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
         P->mucamask |= (op == SU2GPU_PHISQ || op == SU2GPU_PHI2MINUSSIGMA2 ? 1 : 0) |
                        (op == SU2GPU_PHI2SQ ? 2 : 0) | (op == SU2GPU_SIGMASQ || op == SU2GPU_PHI2MINUSSIGMA2 ? 4 : 0);
       }
+    }
     P->nmuca = (int)ms.size();
+    P->h_mfirst.push_back(P->nmuca);
     // restore blocks per chain: up to 8 sites per thread
     P->restore_kb = (int)std::max<int64_t>(1, (mhalf + 8 * 128 - 1) / (8 * 128));
     if (int rc = P->mslots.ensure(std::max<size_t>(ms.size(), 1) * sizeof(int))) return rc;
@@ -403,13 +439,20 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
     // the grouped mode (set by the autotuner or su2gpu_pool_set_sweep_groups)
     // takes precedence over the automatic choice, not over a forced one
     P->grouped = P->grp_G > 1 && (int)P->active.size() > 1 && P->persist_mode != 1 && P->nmuca == 0;
+    P->run_NS = P->grp_NS;
+    P->h_groups.clear();
     if (P->grouped) {
       P->persistent = false;
       P->h_groups = make_groups(P, P->grp_G, false);
-    } else {
-      P->h_groups.clear();
     }
     if (int rc = choose_teams(P, fits)) return rc;
+    if (fits) choose_groups(P);  // a long recipe keeps one launch per pass
+    if (P->grouped || P->team) {  // not first in a sweep, whose stream may be capturing
+      std::vector<cudaStream_t> ss;
+      const int ns = std::max(P->run_NS, (int)P->teams.size());
+      if (int rc = sweep_streams(P, ns, ss)) return rc;
+      if (int rc = ensure_events(P->grp_ev, (size_t)ns + 1)) return rc;
+    }
     P->h_segs.clear();
     P->h_sfirst.clear();
     for (int s : P->active) {
@@ -513,9 +556,13 @@ void sweep_recipe(const su2gpu_params& p, std::vector<PassDesc>& out, int64_t* t
   }
 }
 
-// one sweep of every chain of the tile tables, one launch per pass
+// one sweep of the active chains [a0, a1) (default: all), whose tiles are the
+// tables given, one launch per pass
 int enqueue_pool_sweep(su2gpu_pool* P, const void* descs, const int2* const* tiles, const int* nt,
-                       int64_t* tot) {
+                       int64_t* tot, int a0 = 0, int a1 = -1) {
+  if (a1 < 0) a1 = (int)P->active.size();
+  const int* mslots = (const int*)P->mslots.p + P->h_mfirst[a0];
+  const int nm = P->h_mfirst[a1] - P->h_mfirst[a0];
   if (!nt) nt = P->ntiles;
   std::vector<PassDesc> passes;
   sweep_recipe(P->recipe, passes, tot, P->mucamask);
@@ -531,8 +578,8 @@ int enqueue_pool_sweep(su2gpu_pool* P, const void* descs, const int2* const* til
     mark(P, kind);
     if (kind == 0) P->pers->pool_link(v, a, nt[v], P->st);
     else if (kind == 1) P->pers->pool_u1(v, a, nt[v], P->st);
-    else if (kind == 5) P->pers->pool_restore(a, (const int*)P->mslots.p, P->nmuca, P->restore_kb, P->st);
-    else if (kind == 6) P->pers->pool_decide(a, (const int*)P->mslots.p, P->nmuca, P->st);
+    else if (kind == 5) P->pers->pool_restore(a, mslots, nm, P->restore_kb, P->st);
+    else if (kind == 6) P->pers->pool_decide(a, mslots, nm, P->st);
     else P->pers->pool_scalar(v, kind - 2, a, nt[v], P->st);
   }
   mark(P, -1);
@@ -1160,30 +1207,37 @@ static int pool_enqueue(su2gpu_pool* P, int32_t nsweeps, int32_t use_graph) {
   } else if (P->team) {
     if ((rc = enqueue_teams(P, sweeps, na, nsweeps, tot))) return rc;
   } else if (P->grouped) {
-    // the groups' sweeps on grp_NS streams in turn, forked from and joined
+    // the groups' sweeps on run_NS streams in turn, forked from and joined
     // back into the pool's stream
     const int Gn = (int)P->h_groups.size() - 1;
     std::vector<cudaStream_t> ss;
-    if ((rc = sweep_streams(P, P->grp_NS, ss)) || (rc = ensure_events(P->grp_ev, ss.size() + 1))) return rc;
+    if ((rc = sweep_streams(P, P->run_NS, ss)) || (rc = ensure_events(P->grp_ev, ss.size() + 1))) return rc;
     const int NS = (int)ss.size();
+    // A group's graph is one sweep, or two where there are many groups,
+    // replayed (384 chains: capturing all ten sweeps of a run made the pool's
+    // first run 10 ms longer, one-sweep graphs the others 0.3 ms).  The replays
+    // of the groups that run side by side are enqueued in turn, and a group's
+    // graph is captured just before its first replay, while the groups before
+    // it already run.
+    const int per = Gn <= 2 * NS || nsweeps % 2 ? 1 : 2;
     std::vector<cudaGraphExec_t> gex(Gn, nullptr);
-    if (use_graph)
-      for (int g = 0; g < Gn; g++)
-        if ((rc = group_graph(P, P->h_groups[g], P->h_groups[g + 1], nsweeps, &gex[g], true))) return rc;
     PCK(cudaEventRecord(P->grp_ev[0], P->st));
     for (int k = 0; k < NS; k++) PCK(cudaStreamWaitEvent(ss[k], P->grp_ev[0], 0));
-    for (int g = 0; g < Gn; g++) {
-      if (use_graph) {
-        PCK(cudaGraphLaunch(gex[g], ss[g % NS]));
-      } else {
-        cudaStream_t home = P->st;
-        P->st = ss[g % NS];
-        int64_t t1[SU2GPU_NCOUNTERS] = {0};
-        rc = enqueue_group_sweep(P, P->h_groups[g], P->h_groups[g + 1], nsweeps, t1, true);
-        P->st = home;
-        if (rc) return rc;
-      }
-    }
+    for (int g0 = 0; g0 < Gn; g0 += NS)
+      for (int k = 0; k < nsweeps; k += per)
+        for (int g = g0; g < std::min(g0 + NS, Gn); g++) {
+          if (use_graph) {
+            if (!gex[g] && (rc = group_graph(P, P->h_groups[g], P->h_groups[g + 1], per, &gex[g], true))) return rc;
+            PCK(cudaGraphLaunch(gex[g], ss[g % NS]));
+          } else {
+            cudaStream_t home = P->st;
+            P->st = ss[g % NS];
+            int64_t t1[SU2GPU_NCOUNTERS] = {0};
+            rc = enqueue_group_sweep(P, P->h_groups[g], P->h_groups[g + 1], per, t1, true);
+            P->st = home;
+            if (rc) return rc;
+          }
+        }
     for (int k = 0; k < NS; k++) {
       PCK(cudaEventRecord(P->grp_ev[k + 1], ss[k]));
       PCK(cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0));
@@ -1276,7 +1330,7 @@ static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* t
   }
   for (int k = 0; k < n; k++) {
     int64_t t1[SU2GPU_NCOUNTERS] = {0};
-    int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot);
+    int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot, a0, a1);
     if (rc) return rc;
     launch_pool_next_sweep(sweeps, a1 - a0, P->st);
   }
@@ -1349,12 +1403,18 @@ static std::vector<int> make_groups(const su2gpu_pool* P, int G, bool light_ends
   return b;
 }
 
-// the cycle's groups: about 64 MB of host arrays each, at most 32
+// The cycle's groups: about 64 MB of host arrays each, at most 32, swept on
+// three streams in turn; a batch of fewer than 8 such groups is cut into up to
+// 8 of 20 MB on up to six streams instead, so that the transfers of most groups
+// and the gaps between most passes are covered (64 chains, 141 MB: 2 groups 2490
+// us, 4 on 4 streams 2325, 6 on 6 2180, 8 on 6 2160, 16 on 6 2590).
+constexpr int SMALL_CYCLE_GROUPS = 8, SMALL_CYCLE_STREAMS = 6;
 static std::vector<int> cycle_groups(const su2gpu_pool* P) {
   int64_t total = 0;
   for (int s : P->active) total += P->slots[s].g.V;
   const int64_t bytes = total * STAGE_REALS * 8;
-  int G = (int)std::min<int64_t>(32, std::max<int64_t>(1, bytes / (64ll << 20)));
+  int G = (int)std::min<int64_t>(32, bytes / (64ll << 20));
+  if (G < SMALL_CYCLE_GROUPS) G = (int)std::min<int64_t>(SMALL_CYCLE_GROUPS, std::max<int64_t>(1, bytes / (20ll << 20)));
   const char* e = getenv("SU2GPU_CYCLE_GROUPS");
   if (e && *e) G = std::max(1, atoi(e));
   return make_groups(P, G, true);
@@ -1412,7 +1472,7 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
   // blocks, each pass with its ramp and tail) run on NS streams in turn, so
   // that consecutive groups fill each other's gaps; persistent groups share
   // the work counters and stay on one stream
-  int NS = any_persistent ? 1 : std::min(G, 3);
+  int NS = any_persistent ? 1 : std::min(G, G <= SMALL_CYCLE_GROUPS ? SMALL_CYCLE_STREAMS : 3);
   if (const char* e = getenv("SU2GPU_CYCLE_STREAMS"); e && *e && !any_persistent)
     NS = std::max(1, std::min(std::min(G, su2gpu_pool::CYCLE_SWEEP_STREAMS), atoi(e)));
   std::vector<cudaStream_t> ss;
@@ -1766,7 +1826,7 @@ int su2gpu_pool_get_sweep_groups(su2gpu_pool* P, int32_t* groups, int32_t* strea
   int rc;
   if (P->dirty && (rc = rebuild(P))) return rc;
   *groups = P->grouped ? (int)P->h_groups.size() - 1 : 0;
-  *streams = P->grouped ? std::min(P->grp_NS, su2gpu_pool::CYCLE_SWEEP_STREAMS) : 1;
+  *streams = P->grouped ? std::min(P->run_NS, su2gpu_pool::CYCLE_SWEEP_STREAMS) : 1;
   return SU2GPU_OK;
 }
 
@@ -1892,7 +1952,7 @@ static int time_grouped(su2gpu_pool* P, void* descs, int G, int NS, int reps, fl
     int64_t t1[SU2GPU_NCOUNTERS] = {0};
     cudaError_t e = cudaStreamBeginCapture(P->st, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      for (int k = 0; k < TUNE_SWEEPS && !rc; k++) rc = enqueue_pool_sweep(P, descs, tiles, nt, t1);
+      for (int k = 0; k < TUNE_SWEEPS && !rc; k++) rc = enqueue_pool_sweep(P, descs, tiles, nt, t1, groups[g], groups[g + 1]);
       e = cudaStreamEndCapture(P->st, &graph);
       if (e == cudaSuccess) {
         e = cudaGraphInstantiate(&gex[g], graph, 0);
@@ -2092,7 +2152,10 @@ int su2gpu_pool_autotune(su2gpu_pool* P, int32_t* choices, float* best_ms) {
       }
       if (!rc) base_ms = ms / reps / TUNE_SWEEPS;
     }
-    if (!rc && base_ms <= 0.f && (rc = time_grouped(P, desc2.p, 1, 1, reps, &base_ms))) {
+    // the automatic choice's groups, or one launch per pass
+    const bool own = P->grouped && P->grp_G <= 1;
+    if (!rc && base_ms <= 0.f &&
+        (rc = time_grouped(P, desc2.p, own ? (int)P->h_groups.size() - 1 : 1, own ? P->run_NS : 1, reps, &base_ms))) {
       // base_ms stays unset; rc is returned below
     }
     // (groups, streams): on the 384-chain ensemble (11 M sites) groups of
