@@ -218,9 +218,9 @@ __device__ inline double mexp(double x) { return exp(x); }
 __device__ inline float mexp(float x) { return expf(x); }
 __device__ inline double mcos(double x) { return cos(x); }
 __device__ inline float mcos(float x) { return cosf(x); }
-// cos(2 pi u) for u in [0,1): FP64 keeps the reference's cos(2*M_PI*u)
-// (heatbath.c:56); FP32 uses cospi, which needs no argument reduction
-__device__ inline double mcos2pi(double u) { return cos(2 * 3.14159265358979323846 * u); }
+// cos(2 pi u) for u in [0,1) (heatbath.c:56) by cospi, which needs no argument
+// reduction
+__device__ inline double mcos2pi(double u) { return cospi(2.0 * u); }
 __device__ inline float mcos2pi(float u) { return cospif(2.0f * u); }
 __device__ inline double msin(double x) { return sin(x); }
 __device__ inline float msin(float x) { return sinf(x); }

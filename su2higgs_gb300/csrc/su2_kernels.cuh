@@ -424,13 +424,13 @@ __device__ inline int heatbath(const Fields<R>& f, const Geom& g, const CoupT<R>
     oldact = hop_triplet_fwd_u(f, g, c, i, mu, old);
   }
   Q<R> V = link_staple<R, CC>(f, g, cp, c, i, mu);
-  R a = msqrt(qsq(V));
-  R ia = 0;  // FP64: 1 / (2 |V|), the one division by the staple's length
+  R a = 0, ia = 0;  // FP64 uses ia = 1 / (2 |V|), one reciprocal square root
   if constexpr (sizeof(R) == 8) {
-    ia = (R)1 / a;
+    ia = rsqrt(qsq(V));
     V = qscale(V, -ia);
     ia *= (R)0.5;
   } else {
+    a = msqrt(qsq(V));
     V = qscale(V, (R)-1 / a);
     a *= (R)2;
   }
@@ -483,7 +483,7 @@ __device__ inline int heatbath(const Fields<R>& f, const Geom& g, const CoupT<R>
         return 0;
       }
     }
-    d = rad / msqrt(d);
+    d = rad * rsqrt(d);
     nl = Q<R>{a0, r1 * d, r2 * d, r3 * d};
   } else {
     // FP32 form: the same uniform direction drawn directly (Archimedes:
@@ -618,7 +618,7 @@ __device__ inline int overrelax_f64(double (&p)[N], const double (&s)[N], double
     ss += s[k] * s[k];
     ps += p[k] * s[k];
   }
-  const double F = sqrt(ss), iF = 1.0 / F, X = ps * iF;
+  const double iF = rsqrt(ss), F = ss * iF, X = ps * iF;
 #pragma unroll
   for (int k = 0; k < N; k++) {
     const double y = p[k] - X * iF * s[k];
