@@ -1902,8 +1902,8 @@ __global__ void k_reduce_partials(const double* partials, int np, double* out) {
 // gradient flow (gradflow.c:190-414): forces from `in`, Euler step into `out`
 // ---------------------------------------------------------------------------
 template <typename R, int CC>
-__global__ void __launch_bounds__(BLOCK) k_flow(Fields<R> in, Fields<R> out, Geom g, CoupT<R> cp, R dt,
-                                                unsigned long long* first_zero) {
+__device__ inline void flow_site(const Fields<R>& in, const Fields<R>& out, const Geom& g, const CoupT<R>& cp, R dt,
+                                 unsigned long long* first_zero) {
   int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.V) return;
   int parity = t >= g.half;
@@ -1967,16 +1967,35 @@ __global__ void __launch_bounds__(BLOCK) k_flow(Fields<R> in, Fields<R> out, Geo
   }
 }
 
-// links at or after the first zero-force link keep their value (the
-// reference's early return in flow_gauge)
-template <typename R>
-__global__ void k_flow_fixup(Fields<R> in, Fields<R> out, Geom g, const unsigned long long* first_zero) {
-  unsigned long long fz = *first_zero;
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.V * 3 || (unsigned long long)t < fz) return;
-  int i = t / 3;
-  int mu = (int)(t - i * 3);
-  lk(out, mu)[i] = lk(in, mu)[i];
+// One Euler step.  Links at or after the first zero-force link keep their value
+// (the reference's early return in flow_gauge): the block that finishes last
+// puts them back -- usually there is none, and it only sets the marker and the
+// arrival count for the next step.  (A kernel that reset the marker and one that
+// looked at it were two launches a step.)
+template <typename R, int CC>
+__global__ void __launch_bounds__(BLOCK) k_flow(Fields<R> in, Fields<R> out, Geom g, CoupT<R> cp, R dt,
+                                                unsigned long long* first_zero, unsigned* arrive) {
+  __shared__ int s_last;
+  flow_site<R, CC>(in, out, g, cp, dt, first_zero);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(arrive, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const unsigned long long fz = *(volatile unsigned long long*)first_zero;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *first_zero = ~0ull;
+    *arrive = 0;
+  }
+  if (fz == ~0ull) return;
+  for (unsigned long long t = fz + threadIdx.x; t < 3ull * (unsigned long long)g.V; t += BLOCK) {
+    const int i = (int)(t / 3), mu = (int)(t - 3ull * (unsigned long long)i);
+    lk(out, mu)[i] = lk(in, mu)[i];
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -60,7 +60,6 @@ __global__ void k_inc_u32(uint32_t* p) {
   dependent_wait();
   *p += 1u;
 }
-__global__ void k_fill_u64(unsigned long long* p, unsigned long long v) { *p = v; }
 
 // layout tables (layout.c:657-756 serial order) from the closed form
 __global__ void k_layout_tables(Geom g, int64_t* next, int64_t* prev, int64_t* coords, int32_t* parity) {
@@ -1218,14 +1217,15 @@ static int flow_impl(su2gpu_ctx* c, Fields<R>& main, double t_max, double dt, in
     return SU2GPU_OK;
   };
   if ((rc = meas(t))) return rc;
+  // the first zero-force link's marker and the blocks' arrival count, which
+  // every step leaves as it found them
+  CK(cudaMemsetAsync(c->d_fz, 0xff, 8, c->st));
+  CK(cudaMemsetAsync(c->d_fz + 1, 0, 4, c->st));
   int iter = 1;
   unsigned nb = nblk(V, BLOCK);
   while (t < t_max) {
     if (t + dt > t_max) dt = t_max - t;
-    k_fill_u64<<<1, 1, 0, c->st>>>(c->d_fz, ~0ull);
-    c->ops->flow(&A, &B, c->g, cp, dt, c->d_fz, nb, c->st);
-    CKL();
-    c->pops->flow_fixup(&A, &B, c->g, c->d_fz, c->st);
+    c->ops->flow(&A, &B, c->g, cp, dt, c->d_fz, (unsigned*)(c->d_fz + 1), nb, c->st);
     CKL();
     std::swap(A, B);
     t += dt;
