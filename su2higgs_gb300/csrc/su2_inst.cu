@@ -17,23 +17,22 @@ using R = SU2_R;
 constexpr int CCI = SU2_CC;
 
 // Threads per block of an update launch over n sites.  FP64: a launch of few
-// warps is cut into blocks of one warp (two where the launch decides a
-// multicanonical check, whose sums take 64 threads), so that no SM quarter has
-// more warps than the others: the FP64 pipe (half a lane a cycle and quarter: a
+// warps is cut into blocks of one warp, so that no SM quarter has more warps
+// than the others: the FP64 pipe (half a lane a cycle and quarter: a
 // warp instruction holds it for 64 cycles, 76 with the three neighbours busy)
 // is the bound; 16^3 doublet half-sweep 14.9 -> 12.6 us.  Past 16 warps an SM
 // whole blocks balance as well.  FP32 warps hide each other's latency and share
 // their SM's L1: blocks of one warp cost 2-5 % there at every size tried
 // (42 x 12 x 30 to 88 x 72 x 14).
-static unsigned launch_threads(int n, int bs, bool check) {
+static unsigned launch_threads(int n, int bs) {
   if (sizeof(R) == 4 || (n + 31) / 32 > 152 * 16) return (unsigned)bs;
-  return (unsigned)std::min(bs, check ? 64 : 32);
+  return (unsigned)std::min(bs, 32);
 }
 
 template <int V>
 static unsigned l_link_v(const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
-  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS, false);
+  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS);
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
@@ -45,7 +44,7 @@ static unsigned l_link_v(const void* f, const PassArgs& a, cudaStream_t st) {
 template <int V>
 static unsigned l_u1_v(const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
-  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS, false);
+  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS);
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
@@ -57,7 +56,7 @@ static unsigned l_u1_v(const void* f, const PassArgs& a, cudaStream_t st) {
 template <int V>
 static unsigned l_scalar_v(int field, const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
-  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS, a.muca != nullptr);
+  const unsigned bs = launch_threads(a.t_hi - a.t_lo, BS);
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
@@ -123,6 +122,17 @@ static void p_restore(int field, const void* f, const MucaDev* m, const void* ba
   else
     launch_dependent(k_muca_restore<R, 1>, nb, 256, st, *(const Fields<R>*)f, m, backup, h, (int)lo, (int)hi);
 }
+static void p_muca_finish(int field, const void* f, MucaDev* w, const double* partials, int np, double vol, int parity,
+                          const RngKey& rk, uint32_t pass, uint32_t check, unsigned long long* ctr, const void* backup,
+                          int h, int lo, int hi, unsigned* arrive, cudaStream_t st) {
+  const unsigned nb = std::min<unsigned>(nblk(hi - lo, 256), MUCA_FINISH_BLOCKS);
+  if (field == 0)
+    launch_dependent(k_muca_finish<R, 0>, nb, 256, st, *(const Fields<R>*)f, w, partials, np, vol, parity, rk, pass, check,
+                     ctr, backup, h, lo, hi, arrive);
+  else
+    launch_dependent(k_muca_finish<R, 1>, nb, 256, st, *(const Fields<R>*)f, w, partials, np, vol, parity, rk, pass, check,
+                     ctr, backup, h, lo, hi, arrive);
+}
 static void p_alpha(const void* f, const Geom& g, const Coup& cp, double* alpha, cudaStream_t st) {
   const unsigned nb = nblk(g.V, BLOCK);
   launch_dependent(k_alpha<R>, nb, BLOCK, st, *(const Fields<R>*)f, g, coup_as<R>(cp), alpha);
@@ -149,7 +159,7 @@ static void p_pool_convert(const void* descs, const ConvItem* items, int n, int 
   dim3 grid(std::min(nblk(vmax, 256), 128u), (unsigned)n);
   k_pool_convert<R><<<grid, 256, 0, st>>>(descs, items, staging, to_device);
 }
-const PrecOps SU2_WITH_PREC = {p_orderparam, p_restore, p_alpha, p_import, p_export, p_reunit,
+const PrecOps SU2_WITH_PREC = {p_orderparam, p_restore, p_muca_finish, p_alpha, p_import, p_export, p_reunit,
                                p_measure_local, p_measure_z, p_pool_convert};
 #endif
 

@@ -43,6 +43,11 @@ struct PrecOps {
                      cudaStream_t st);
   void (*restore)(int field, const void* f, const MucaDev* m, const void* backup, int h, int64_t lo, int64_t hi,
                   cudaStream_t st);
+  // the check of a whole parity after its update: decision, restore, commit
+  // (k_muca_finish); arrive: a device word that is 0
+  void (*muca_finish)(int field, const void* f, MucaDev* w, const double* partials, int np, double vol, int parity,
+                      const RngKey& rk, uint32_t pass, uint32_t check, unsigned long long* ctr, const void* backup, int h,
+                      int lo, int hi, unsigned* arrive, cudaStream_t st);
   void (*alpha)(const void* f, const Geom& g, const Coup& cp, double* alpha, cudaStream_t st);
   void (*import)(const void* f, int64_t V, int kind, int h, const double* src, cudaStream_t st);
   void (*exportf)(const void* f, int64_t V, int kind, int h, double* dst, cudaStream_t st);
