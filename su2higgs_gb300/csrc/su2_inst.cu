@@ -29,6 +29,12 @@ static unsigned launch_threads(int n, int bs) {
   return (unsigned)std::min(bs, 32);
 }
 
+// blocks of a split pass over n sites, 0 where passes are not split
+static unsigned split_blocks(int n) {
+  const unsigned nb = (unsigned)(n + 31) / 32;
+  return sizeof(R) == 8 && nb <= SPLIT_GROUPS ? nb : 0;
+}
+
 template <int V>
 static unsigned l_link_v(const void* f, const PassArgs& a, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
@@ -36,6 +42,15 @@ static unsigned l_link_v(const void* f, const PassArgs& a, cudaStream_t st) {
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
+  if constexpr (sizeof(R) == 8) {
+    const unsigned ns = a.alg == ALG_HEATBATH ? split_blocks(a.t_hi - a.t_lo) : 0;
+    if (ns) {
+      if (a.sub == 0) launch_dependent(k_link_split<CCI, 0>, ns, 128, st, F, a);
+      else if (a.sub == 1) launch_dependent(k_link_split<CCI, 1>, ns, 128, st, F, a);
+      else launch_dependent(k_link_split<CCI, 2>, ns, 128, st, F, a);
+      return ns;
+    }
+  }
   if (a.sub == 0) launch_dependent(k_link<R, CCI, 0, BS, MB>, nb, bs, st, F, a);
   else if (a.sub == 1) launch_dependent(k_link<R, CCI, 1, BS, MB>, nb, bs, st, F, a);
   else launch_dependent(k_link<R, CCI, 2, BS, MB>, nb, bs, st, F, a);
@@ -60,6 +75,14 @@ static unsigned l_scalar_v(int field, const void* f, const PassArgs& a, cudaStre
   unsigned nb = ((unsigned)(a.t_hi - a.t_lo) + bs - 1) / bs;
   if (!nb) return 0;
   const Fields<R>& F = *(const Fields<R>*)f;
+  if constexpr (sizeof(R) == 8) {
+    const unsigned ns = field < 2 ? split_blocks(a.t_hi - a.t_lo) : 0;
+    if (ns) {
+      if (field == 0) launch_dependent(k_scalar_split<CCI, 0>, ns, 128, st, F, a);
+      else launch_dependent(k_scalar_split<CCI, 1>, ns, 128, st, F, a);
+      return ns;
+    }
+  }
   if (field == 0) launch_dependent(k_scalar<R, CCI, 0, BS, MB>, nb, bs, st, F, a);
   else if (field == 1) launch_dependent(k_scalar<R, CCI, 1, BS, MB>, nb, bs, st, F, a);
   else launch_dependent(k_scalar<R, CCI, 2, BS, MB>, nb, bs, st, F, a);

@@ -591,11 +591,10 @@ __device__ inline int metro_u1_f64(const Fields<double>& f, const Geom& g, const
 // field, so dS = (p'-p).s + 3 (p'^2-p^2) + V(p') - V(p) with s =
 // staple_doublet -- the neighbours are multiplied once instead of four times
 template <int CC>
-__device__ inline int metro_doublet_f64(const Fields<double>& f, const Geom& g, const CoupT<double>& cp, const int* c,
-                                        int i, int h, SiteRng<double>& rng) {
+__device__ inline int metro_doublet_f64(const Fields<double>& f, const CoupT<double>& cp, int i, int h,
+                                        const Q<double>& s, SiteRng<double>& rng) {
   using R = double;
   const R d0 = rng.uni() - 0.5, d1 = rng.uni() - 0.5, d2 = rng.uni() - 0.5, d3 = rng.uni() - 0.5;
-  const Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, h);
   const Q<R> old = ld4<R>(php(f, h), i), nw{old.a + d0, old.b + d1, old.c + d2, old.d + d3};
   const Q<R> e{nw.a - old.a, nw.b - old.b, nw.c - old.c, nw.d - old.d};
   const R dsq = e.a * (nw.a + old.a) + e.b * (nw.b + old.b) + e.c * (nw.c + old.c) + e.d * (nw.d + old.d);
@@ -635,6 +634,48 @@ __device__ inline int overrelax_f64(double (&p)[N], const double (&s)[N], double
   return 1;
 }
 
+// the doublet's (one doublet) and the triplet's, with their staples s
+template <int CC>
+__device__ inline int overrelax_doublet_f64(const Fields<double>& f, const CoupT<double>& cp, int i,
+                                            const Q<double>& s, double u, int* fallback) {
+  const Q<double> p = ld4<double>(php(f, 0), i);
+  double B = 0.5 * cp.msq + 3.0;
+  if (HAS(C_T)) B += 0.5 * cp.a2 * tripletsq(ld3(f, i));
+  if (HAS(C_S)) {
+    const double S = f.sing[i];
+    B += 0.25 * cp.a1s * S + 0.25 * cp.a2s * S * S;
+  }
+  const double sv[4] = {s.a, s.b, s.c, s.d};
+  double pv[4] = {p.a, p.b, p.c, p.d};
+  if (!overrelax_f64<4>(pv, sv, B, 0.25 * cp.lam, u, fallback)) return 0;
+  st4<double>(php(f, 0), i, Q<double>{pv[0], pv[1], pv[2], pv[3]});
+  return 1;
+}
+__device__ inline int overrelax_triplet_f64(const Fields<double>& f, const CoupT<double>& cp, int i,
+                                            const V3<double>& s, double u, int* fallback) {
+  const V3<double> t = ld3(f, i);
+  const double sv[3] = {s.x, s.y, s.z};
+  double tv[3] = {t.x, t.y, t.z};
+  if (!overrelax_f64<3>(tv, sv, 0.5 * cp.msqT + 3.0, 0.25 * cp.b4, u, fallback)) return 0;
+  st3(f, i, V3<double>{tv[0], tv[1], tv[2]});
+  return 1;
+}
+// metro_triplet's FP64 form with its staple s (see metro_triplet)
+template <int CC>
+__device__ inline int metro_triplet_f64(const Fields<double>& f, const CoupT<double>& cp, int i, const V3<double>& s,
+                                        SiteRng<double>& rng) {
+  const double dx = rng.uni() - 0.5, dy = rng.uni() - 0.5, dz = rng.uni() - 0.5;
+  const V3<double> old = ld3(f, i), nw{old.x + dx, old.y + dy, old.z + dz};
+  const double ex = nw.x - old.x, ey = nw.y - old.y, ez = nw.z - old.z;
+  const double dsq = ex * (nw.x + old.x) + ey * (nw.y + old.y) + ez * (nw.z + old.z);
+  const double ssq = (nw.x * nw.x + nw.y * nw.y + nw.z * nw.z) + (old.x * old.x + old.y * old.y + old.z * old.z);
+  double B = 0.5 * cp.msqT + 3.0;
+  if (NHIGGS > 0) B += 0.5 * cp.a2 * doubletsq(ld4<double>(php(f, 0), i));
+  if (!metro_accept(ex * s.x + ey * s.y + ez * s.z + dsq * (B + 0.25 * cp.b4 * ssq), rng)) return 0;
+  st3(f, i, nw);
+  return 1;
+}
+
 // metro_u1link (metropolis.c:48-70)
 template <typename R, int CC>
 __device__ inline int metro_u1(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i, int mu,
@@ -653,7 +694,8 @@ __device__ inline int metro_u1(const Fields<R>& f, const Geom& g, const CoupT<R>
 template <typename R, int CC>
 __device__ inline int metro_doublet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                     int h, SiteRng<R>& rng) {
-  if constexpr (sizeof(R) == 8) return metro_doublet_f64<CC>(f, g, cp, c, i, h, rng);
+  if constexpr (sizeof(R) == 8)
+    return metro_doublet_f64<CC>(f, cp, i, h, staple_doublet<R, CC>(f, g, cp, c, i, h), rng);
   const R d0 = rng.uni() - (R)0.5, d1 = rng.uni() - (R)0.5, d2 = rng.uni() - (R)0.5, d3 = rng.uni() - (R)0.5;
   Q<R> old = ld4<R>(php(f, h), i);
   R a0 = localact_doublet<R, CC>(f, g, cp, c, i, h);
@@ -674,20 +716,8 @@ template <typename R, int CC, typename RNG>
 __device__ inline int overrelax_doublet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                         RNG& rng, int* fallback) {
   const R u = rng.uni();
-  if constexpr (sizeof(R) == 8) {
-    const Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, 0), p = ld4<R>(php(f, 0), i);
-    R B = 0.5 * cp.msq + 3.0;
-    if (HAS(C_T)) B += 0.5 * cp.a2 * tripletsq(ld3(f, i));
-    if (HAS(C_S)) {
-      const R S = f.sing[i];
-      B += 0.25 * cp.a1s * S + 0.25 * cp.a2s * S * S;
-    }
-    const R sv[4] = {s.a, s.b, s.c, s.d};
-    R pv[4] = {p.a, p.b, p.c, p.d};
-    if (!overrelax_f64<4>(pv, sv, B, 0.25 * cp.lam, u, fallback)) return 0;
-    st4<R>(php(f, 0), i, Q<R>{pv[0], pv[1], pv[2], pv[3]});
-    return 1;
-  }
+  if constexpr (sizeof(R) == 8)
+    return overrelax_doublet_f64<CC>(f, cp, i, staple_doublet<R, CC>(f, g, cp, c, i, 0), u, fallback);
   Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, 0);
   Q<R> p = ld4<R>(php(f, 0), i);
   R F = msqrt(s.a * s.a + s.b * s.b + s.c * s.c + s.d * s.d);
@@ -724,9 +754,11 @@ __device__ inline int overrelax_doublet(const Fields<R>& f, const Geom& g, const
 // overrelax_higgs2 (overrelax.c:295-417)
 template <typename R, int CC, typename RNG>
 __device__ inline int overrelax_higgs2(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
-                                       int h, RNG& rng, int* fallback) {
+                                       int h, RNG& rng, int* fallback, const Q<R>* given = nullptr) {
   const R u = rng.uni();
-  Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, h);
+  Q<R> s;
+  if constexpr (sizeof(R) == 8) s = given ? *given : staple_doublet<R, CC>(f, g, cp, c, i, h);
+  else s = staple_doublet<R, CC>(f, g, cp, c, i, h);
   Q<R> fv = ld4<R>(php(f, h), i);
   Q<R> H;
   R l67re, l67im, lore, loim, lam12, msq;
@@ -811,14 +843,8 @@ template <typename R, int CC, typename RNG>
 __device__ inline int overrelax_triplet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                         RNG& rng, int* fallback) {
   const R u = rng.uni();
-  if constexpr (sizeof(R) == 8) {
-    const V3<R> s = staple_triplet(f, g, c, i), t = ld3(f, i);
-    const R sv[3] = {s.x, s.y, s.z};
-    R tv[3] = {t.x, t.y, t.z};
-    if (!overrelax_f64<3>(tv, sv, 0.5 * cp.msqT + 3.0, 0.25 * cp.b4, u, fallback)) return 0;
-    st3(f, i, V3<R>{tv[0], tv[1], tv[2]});
-    return 1;
-  }
+  if constexpr (sizeof(R) == 8)
+    return overrelax_triplet_f64(f, cp, i, staple_triplet(f, g, c, i), u, fallback);
   V3<R> s = staple_triplet(f, g, c, i);
   V3<R> t = ld3(f, i);
   R F = msqrt(s.x * s.x + s.y * s.y + s.z * s.z);
@@ -854,6 +880,7 @@ __device__ inline int overrelax_triplet(const Fields<R>& f, const Geom& g, const
 template <typename R, int CC>
 __device__ inline int metro_triplet(const Fields<R>& f, const Geom& g, const CoupT<R>& cp, const int* c, int i,
                                     SiteRng<R>& rng) {
+  if constexpr (sizeof(R) == 8) return metro_triplet_f64<CC>(f, cp, i, staple_triplet(f, g, c, i), rng);
   const R e0 = rng.uni() - (R)0.5, e1 = rng.uni() - (R)0.5, e2 = rng.uni() - (R)0.5;
   // FP32: the decision's uniform is the fourth word of the same generator
   // block, drawn with the proposal; FP64 draws it only when it is needed
@@ -1058,6 +1085,247 @@ __global__ void __launch_bounds__(BS, MINB) k_scalar(Fields<R> f, PassArgs a) {
   if (a.partials) {
     double s = block_sum(opv);
     if (threadIdx.x == 0) a.partials[blockIdx.x] = s;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Split passes, the FP64 form of small lattices: a site's update by four lanes,
+// the same lane of the four warps of a block, which run on the four quarters of
+// an SM.  A quarter's FP64 pipe takes a warp instruction in 64 cycles however
+// many lanes or warps there are, so a pass of fewer warps of sites than there are
+// quarters (608) lasts as long as one site's FP64 instructions.  Each warp takes
+// a part of the staple (and of the random numbers' functions); the first goes on
+// with the sum.  Sweep + measurement of the fundamental theory, one lane a site
+// against four: 16^3 (64 groups of 32 sites) 261 / 213 us, 32^3 (512 groups, where
+// the quarters are nearly full) 299 / 306 us; the line lies between.
+// ---------------------------------------------------------------------------
+constexpr int SPLIT_GROUPS = 384;
+
+// draw n of the site's stream
+__device__ inline double draw_at(SiteRng<double>& rng, uint32_t n) {
+  rng.draw = n & ~1u;
+  const double v = rng.uni();
+  return (n & 1u) ? rng.uni() : v;
+}
+
+// Link heatbath (see heatbath).  Before the barrier: warp w computes one of the
+// four products of the Wilson staple; warp 1 the logarithms of the first trial,
+// warp 2 the direction drawn after it, warp 3 its cosine and the doublets' term.
+// A first trial that is rejected (1-2 %) is followed by the others in warp 0.
+template <int CC, int MU>
+__global__ void __launch_bounds__(128) k_link_split(Fields<double> f, PassArgs a) {
+  using R = double;
+  constexpr int N0 = MU == 0 ? 1 : 0, N1 = MU == 2 ? 1 : 2;
+  __shared__ double s_st[5][4][32], s_log[2][32], s_cos[32], s_n[3][32];
+  __shared__ int s_nd[32];
+  dependent_wait();
+  const CoupT<R>& cp = coup<R>(a);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = a.t_lo + (int)blockIdx.x * 32 + lane;
+  const bool on = t < a.t_hi;
+  int c[3];
+  site_coords(a.g, a.parity, on ? t : a.t_lo, c);
+  const Geom& g = a.g;
+  const int i = a.parity * g.half + (on ? t : a.t_lo);
+  SiteRng<R> rng(a.rk, *a.rk.sweep, (uint32_t)i, a.pass);
+  const int xp = shifted(g, c, MU, 1);
+  const int nh = NHIGGS;
+  auto put = [&](int k, const Q<R>& q) {
+    s_st[k][0][lane] = q.a; s_st[k][1][lane] = q.b; s_st[k][2][lane] = q.c; s_st[k][3][lane] = q.d;
+  };
+  {
+    const int nu = w < 2 ? N0 : N1;
+    Q<R> q;
+    if ((w & 1) == 0) {
+      const int xn = shifted(g, c, nu, 1);
+      q = qmul(qmul(ld4<R>(lk(f, nu), xp), qdag(ld4<R>(lk(f, MU), xn))), qdag(ld4<R>(lk(f, nu), i)));
+    } else {
+      const int xpm = shifted(g, c, MU, 1, nu, -1), xm = shifted(g, c, nu, -1);
+      q = qmul(qmul(qdag(ld4<R>(lk(f, nu), xpm)), qdag(ld4<R>(lk(f, MU), xm))), ld4<R>(lk(f, nu), xm));
+    }
+    put(w, q);
+  }
+  R oldact = 0;
+  Q<R> old{};
+  if (w == 0) {
+    if (HAS(C_T)) {
+      old = ld4<R>(lk(f, MU), i);
+      oldact = hop_triplet_fwd_u(f, g, c, i, MU, old);
+    }
+  } else if (w == 1) {
+    const R u0 = rng.uni(), u1 = rng.uni();
+    s_log[0][lane] = -log(1.0 - u0);
+    s_log[1][lane] = -log(1.0 - u1);
+  } else if (w == 2) {
+    rng.draw = 4;
+    R d = 2, r1 = 0, r2 = 0, r3 = 0;
+    int it = 0;
+    while ((d > 1.0 || d == 0.0) && it <= 4096) {
+      r1 = 2.0 * rng.uni() - 1.0;
+      r2 = 2.0 * rng.uni() - 1.0;
+      r3 = 2.0 * rng.uni() - 1.0;
+      d = r1 * r1 + r2 * r2 + r3 * r3;
+      it++;
+    }
+    const R k = rsqrt(d);
+    s_n[0][lane] = r1 * k;
+    s_n[1][lane] = r2 * k;
+    s_n[2][lane] = r3 * k;
+    s_nd[lane] = it > 4096 ? -1 : 4 + 3 * it;  // draws used, -1: none was found
+  } else {
+    const R cs = mcos2pi(draw_at(rng, 2));
+    s_cos[lane] = cs * cs;
+    Q<R> m{0.0, 0.0, 0.0, 0.0};
+    for (int h = 0; h < nh; h++) {
+      Q<R> nphi = ld4<R>(php(f, h), xp);
+      if (HAS(C_U1)) nphi = qphase(nphi, a1p(f, MU)[i]);
+      m = qadd(m, qmul(nphi, qdag(ld4<R>(php(f, h), i))));
+    }
+    put(4, m);
+  }
+  __syncthreads();
+  int acc = 0, cap = 0, err = 0;
+  if (w == 0 && on) {
+    auto get = [&](int k) {
+      return Q<R>{s_st[k][0][lane], s_st[k][1][lane], s_st[k][2][lane], s_st[k][3][lane]};
+    };
+    Q<R> V = qscale(qadd(qadd(get(0), get(1)), qadd(get(2), get(3))), -0.5 * cp.beta);
+    if (nh > 0) {
+      const Q<R> m = get(4);
+      V = Q<R>{V.a - 0.5 * m.a, V.b - 0.5 * m.b, V.c - 0.5 * m.c, V.d - 0.5 * m.d};
+    }
+    R ia = rsqrt(qsq(V));
+    V = qscale(V, -ia);
+    ia *= 0.5;
+    R d = (s_log[0][lane] * s_cos[lane] + s_log[1][lane]) * ia;
+    R r3 = 1.0 - draw_at(rng, 3);
+    int trials = 1;
+    bool ok = r3 * r3 <= 1.0 - 0.5 * d;
+    while (!ok && trials < 200) {
+      const uint32_t n = 4u * (uint32_t)trials;
+      const R u0 = draw_at(rng, n), u1 = rng.uni(), cs = mcos2pi(rng.uni());
+      r3 = 1.0 - rng.uni();
+      d = (-log(1.0 - u0) * (cs * cs) - log(1.0 - u1)) * ia;
+      trials++;
+      ok = r3 * r3 <= 1.0 - 0.5 * d;
+    }
+    R a0 = 1.0 - d;
+    if (trials >= 200) {  // the loop's cap, even if the last trial succeeded
+      a0 = 1e-9;
+      cap = 1;
+    }
+    R rad = 1.0 - a0 * a0;
+    if (rad >= 0.0) {
+      rad = sqrt(rad);
+      R n1 = s_n[0][lane], n2 = s_n[1][lane], n3 = s_n[2][lane];
+      int nd = s_nd[lane];
+      if (trials > 1) {
+        rng.draw = 4u * (uint32_t)trials;
+        R q = 2;
+        int it = 0;
+        while ((q > 1.0 || q == 0.0) && it <= 4096) {
+          n1 = 2.0 * rng.uni() - 1.0;
+          n2 = 2.0 * rng.uni() - 1.0;
+          n3 = 2.0 * rng.uni() - 1.0;
+          q = n1 * n1 + n2 * n2 + n3 * n3;
+          it++;
+        }
+        const R k = rsqrt(q);
+        n1 *= k;
+        n2 *= k;
+        n3 *= k;
+        nd = it > 4096 ? -1 : 4 * trials + 3 * it;
+      }
+      if (nd < 0) {
+        err = 1;
+      } else {
+        const Q<R> U = qmul(Q<R>{a0, n1 * rad, n2 * rad, n3 * rad}, qdag(V));
+        acc = 1;
+        if (HAS(C_T)) acc = draw_at(rng, (uint32_t)nd) < exp(oldact - hop_triplet_fwd_u(f, g, c, i, MU, U));
+        if (acc) st4<R>(lk(f, MU), i, U);
+      }
+    }
+  }
+  dependents_go();
+  if (w == 0) {
+    unsigned long long* ctr = ctr_copy(a.ctr, blockIdx.x);
+    warp_count(ctr + 1, acc);
+    warp_count(ctr + 22, cap);
+    if (err) atomicOr(a.err, 1);
+  }
+}
+
+// a doublet (FIELD 0) or the triplet (1): the six neighbour terms of the staple
+// are one, two, two and one of the warps'
+template <int CC, int FIELD>
+__global__ void __launch_bounds__(128) k_scalar_split(Fields<double> f, PassArgs a) {
+  using R = double;
+  __shared__ double s_st[3][4][32];
+  dependent_wait();
+  const CoupT<R>& cp = coup<R>(a);
+  const Geom& g = a.g;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = FIELD == 0 ? a.sub : 0;
+  const int t = a.t_lo + (int)blockIdx.x * 32 + lane;
+  const bool on = t < a.t_hi;
+  int c[3];
+  site_coords(g, a.parity, on ? t : a.t_lo, c);
+  const int i = a.parity * g.half + (on ? t : a.t_lo);
+  // the sum of terms k of this warp; k = 2 d forward, 2 d + 1 backward
+  Q<R> s{0.0, 0.0, 0.0, 0.0};
+  auto term = [&](int d, bool back) {
+    const int x = shifted(g, c, d, back ? -1 : 1);
+    const Q<R> u = back ? qdag(ld4<R>(lk(f, d), x)) : ld4<R>(lk(f, d), i);
+    if (FIELD == 0) {
+      Q<R> v = qmul(u, ld4<R>(php(f, h), x));
+      if (HAS(C_U1)) v = qphase(v, back ? -a1p(f, d)[x] : a1p(f, d)[i]);
+      s = Q<R>{s.a - v.a, s.b - v.b, s.c - v.c, s.d - v.d};
+    } else {
+      const V3<R> v = qrot(u, ld3(f, x));
+      s = Q<R>{0.0, s.b - v.x, s.c - v.y, s.d - v.z};
+    }
+  };
+  if (w == 0) {
+    term(0, false);
+  } else {
+    if (w == 1) { term(0, true); term(1, false); }
+    else if (w == 2) { term(1, true); term(2, false); }
+    else term(2, true);
+    s_st[w - 1][0][lane] = s.a; s_st[w - 1][1][lane] = s.b; s_st[w - 1][2][lane] = s.c; s_st[w - 1][3][lane] = s.d;
+  }
+  __syncthreads();
+  int acc = 0, fb = 0;
+  double opv = 0.0;
+  const bool orr = (FIELD == 0 ? cp.alg_d : cp.alg_t) == ALG_OR && !a.alg;
+  if (w == 0 && on) {
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      s = Q<R>{s.a + s_st[k][0][lane], s.b + s_st[k][1][lane], s.c + s_st[k][2][lane], s.d + s_st[k][3][lane]};
+    SiteRng<R> rng(a.rk, *a.rk.sweep, (uint32_t)i, a.pass);
+    if (FIELD == 0) {
+      if (a.backup) ((V4<R>*)a.backup)[i] = php(f, h)[i];
+      if (!orr) acc = metro_doublet_f64<CC>(f, cp, i, h, s, rng);
+      else if (NHIGGS == 2) acc = overrelax_higgs2<R, CC>(f, g, cp, c, i, h, rng, &fb, &s);
+      else acc = overrelax_doublet_f64<CC>(f, cp, i, s, rng.uni(), &fb);
+    } else {
+      if (a.backup) {
+        R* b = (R*)a.backup;
+        b[3 * i] = f.trip[0][i]; b[3 * i + 1] = f.trip[1][i]; b[3 * i + 2] = f.trip[2][i];
+      }
+      const V3<R> st{s.b, s.c, s.d};
+      if (orr) acc = overrelax_triplet_f64(f, cp, i, st, rng.uni(), &fb);
+      else acc = metro_triplet_f64<CC>(f, cp, i, st, rng);
+    }
+    if (a.partials) opv = orderparam_site<R>(f, a.op, i);
+  }
+  dependents_go();
+  if (w == 0) {
+    unsigned long long* ctr = ctr_copy(a.ctr, blockIdx.x);
+    warp_count(ctr + (FIELD == 0 ? (orr ? 10 : 6) + a.sub : (orr ? 15 : 13)), acc);
+    warp_count(ctr + 23, fb);
+  }
+  if (a.partials) {
+    const double sum = block_sum(opv);
+    if (threadIdx.x == 0) a.partials[blockIdx.x] = sum;
   }
 }
 
