@@ -271,22 +271,26 @@ void append_segments(const su2gpu_pool* P, int s, int seg, std::vector<int4>& ou
   for (int t0 = 0; t0 < half; t0 += step) out.push_back(int4{s, t0, nseg, 0});
 }
 
-// The team sweep is the automatic choice where every chain fits a team and all
-// teams are resident at once: then each pass of each chain takes its own
-// latency, ~2 us, where a launch per pass takes 4-6 us whatever it covers.  A
-// chain's team: four warps a block (in FP64, one per SM quarter) up to 16
-// blocks, then more threads a block.  FP32 teams end at 16 warps a block (8192
-// sites of a parity, 25^3): beyond, a block's passes take as long as a launch
-// over all SMs.  FP64 warps on one quarter run one after another, so FP64
-// teams end at four warps a block.
-struct TeamShape { int blocks, threads; };
+// The team sweep is the automatic choice where every chain fits a team and the
+// teams leave each other room: then each pass of each chain takes its own
+// latency, ~2 us, where a launch per pass takes 3-6 us whatever it covers.  A
+// chain's team: blocks of four warps (one per SM quarter), up to 16 of them,
+// then more warps a block, up to 8192 sites of a parity (25^3); beyond, a
+// block's passes take as long as a launch over all SMs.  Clusters share SMs
+// long before the SMs are full, so the warps of all teams are limited: 24 FP32
+// chains of 16^3 (1536 warps a pass) take 202 us for four sweeps against 258, of
+// 20^3 (3000) 301 against 286, 6 of 24^3 (1296) 207 against 250, 7 of 24^3 with
+// 21 smaller ones 1454 against 1029.  FP64 warps on one quarter run one after
+// another, so FP64 teams have one warp per quarter in all (6 chains of 12^3 1006
+// against 1077 us, 24 of them, 648 warps, 3144 against 1489).
+struct TeamShape { int blocks, threads, warps; };
+constexpr int TEAM_WARPS = 1600, TEAM_LARGE_WARPS = 1300, TEAM_WARPS_F64 = 608;
 bool team_shape(int prec, int half, TeamShape* t) {
   const int w = (half + 31) / 32;  // warps of a pass
-  if (w <= 16) *t = TeamShape{4, 128};
-  else if (w <= 64) *t = TeamShape{TEAM_BLOCKS, 128};
-  else if (prec == 32 && w <= 128) *t = TeamShape{TEAM_BLOCKS, 256};
-  else if (prec == 32 && w <= 256) *t = TeamShape{TEAM_BLOCKS, TEAM_MAX_THREADS};
-  else return false;
+  if (w > (prec == 32 ? 256 : 64)) return false;
+  const int per = w <= 64 ? 4 : (w <= 128 ? 8 : 16);  // warps of a block
+  const int need = (w + per - 1) / per;
+  *t = TeamShape{need <= 2 ? 2 : (need <= 4 ? 4 : (need <= 8 ? 8 : (need <= 12 ? 12 : TEAM_BLOCKS))), 32 * per, w};
   return true;
 }
 int choose_teams(su2gpu_pool* P, bool fits) {
@@ -294,11 +298,15 @@ int choose_teams(su2gpu_pool* P, bool fits) {
   P->teams.clear();
   if (!fits || P->persist_mode >= 0 || P->grouped || P->persistent || P->active.empty()) return SU2GPU_OK;
   std::vector<std::pair<int, int>> order;  // (shape, slot)
+  int warps = 0, large = 0;
   for (int s : P->active) {
     TeamShape t;
     if (!team_shape(P->prec, P->slots[s].g.half, &t)) return SU2GPU_OK;
     order.push_back({t.blocks * 1024 + t.threads, s});
+    warps += P->prec == 64 ? t.blocks * 4 : t.warps;
+    if (t.warps > 64) large += t.warps;
   }
+  if (warps > (P->prec == 64 ? TEAM_WARPS_F64 : TEAM_WARPS) || large > TEAM_LARGE_WARPS) return SU2GPU_OK;
   std::stable_sort(order.begin(), order.end(), [](auto& a, auto& b) { return a.first > b.first; });
   std::vector<int> slots;
   std::vector<su2gpu_pool::Team> teams;
@@ -309,15 +317,8 @@ int choose_teams(su2gpu_pool* P, bool fits) {
     teams.back().count++;
     slots.push_back(o.second);
   }
-  // the shares of the device that the launches fill have to add up to less
-  // than one (placing clusters of several shapes leaves some room unused)
-  double share = 0.0;
-  for (auto& t : teams) {
-    const int n = P->pers->team_clusters(P->nmuca > 0, t.blocks, t.threads);
-    if (n <= 0) return SU2GPU_OK;
-    share += (double)t.count / n;
-  }
-  if (share > 0.9) return SU2GPU_OK;
+  for (auto& t : teams)
+    if (P->pers->team_clusters(P->nmuca > 0, t.blocks, t.threads) <= 0) return SU2GPU_OK;
   if (int rc = P->teamslots.ensure(slots.size() * sizeof(int))) return rc;
   PCK(cudaMemcpyAsync(P->teamslots.p, slots.data(), slots.size() * sizeof(int), cudaMemcpyHostToDevice, P->st));
   PCK(cudaStreamSynchronize(P->st));  // the list is this function's
@@ -657,10 +658,10 @@ int enqueue_teams(su2gpu_pool* P, uint32_t* const* sweeps, int nchains, int nswe
   for (int k = 0; k < n; k++) {
     const su2gpu_pool::Team& t = P->teams[k];
     A.slots = (const int*)P->teamslots.p + t.first;
-    PCK(P->pers->team(P->nmuca > 0, t.blocks, t.threads, t.count, &A, ss[k]));
+    PCK(P->pers->team(P->nmuca > 0, t.blocks, t.threads, t.count, &A, ss[k % ss.size()]));
   }
   if (n > 1)
-    for (int k = 0; k < n; k++) {
+    for (int k = 0; k < (int)ss.size(); k++) {
       PCK(cudaEventRecord(P->grp_ev[k + 1], ss[k]));
       PCK(cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0));
     }

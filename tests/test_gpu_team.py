@@ -14,7 +14,8 @@ from test_gpu_pool_muca import order_parameter, weight_around
 
 pytestmark = pytest.mark.gpu
 
-# half / 32 warps: < 1, 8, 16, 17 (ragged), 64, 72, 128, 144, 256
+# half / 32 warps: < 1, 8, 16, 17 (ragged), 64, 72, 128, 144, 256: clusters of 2, 2,
+# 4, 8 and 16 blocks of four warps, of 12 and 16 of eight, of 12 and 16 of sixteen
 SIDES = [(2, 2, 4), (8, 8, 8), (16, 8, 8), (6, 18, 10), (16, 16, 16), (16, 16, 18), (16, 16, 32), (16, 18, 32),
          (16, 32, 32)]
 
@@ -38,7 +39,7 @@ def make_pool(gpu, content, precision, sides, persistent):
 
 
 @pytest.mark.parametrize("content", ["adj", "fund", "su2u1s", "higgs2"])
-@pytest.mark.parametrize("precision,sides,shapes", [(32, SIDES, 4), (32, SIDES[:3], 1), (64, SIDES[:5], 2)])
+@pytest.mark.parametrize("precision,sides,shapes", [(32, SIDES, 8), (32, SIDES[:3], 2), (64, SIDES[:5], 4)])
 def test_team_equals_per_pass(gpu, content, precision, sides, shapes):
     a, sa, _ = make_pool(gpu, content, precision, sides, None)
     b, sb, _ = make_pool(gpu, content, precision, sides, False)
