@@ -280,7 +280,7 @@ void append_segments(const su2gpu_pool* P, int s, int seg, std::vector<int4>& ou
 // long before the SMs are full, so the warps of all teams are limited: 24 FP32
 // chains of 16^3 (1536 warps a pass) take 202 us for four sweeps against 258, of
 // 20^3 (3000) 301 against 286, 6 of 24^3 (1296) 207 against 250, 7 of 24^3 with
-// 21 smaller ones 1454 against 1029.  FP64 warps on one quarter run one after
+// 21 smaller ones 1454 against 919.  FP64 warps on one quarter run one after
 // another, so FP64 teams have one warp per quarter in all (6 chains of 12^3 1006
 // against 1077 us, 24 of them, 648 warps, 3144 against 1489).
 struct TeamShape { int blocks, threads, warps; };
