@@ -23,8 +23,9 @@ namespace su2 {
 __device__ inline void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ inline void dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// overlap false: launched normally
 template <typename... P, typename... A>
-inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
+inline void launch_pass(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -33,8 +34,13 @@ inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaSt
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <typename... P, typename... A>
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
+  launch_pass(true, kernel, grid, block, st, static_cast<A&&>(args)...);
 }
 
 }  // namespace su2

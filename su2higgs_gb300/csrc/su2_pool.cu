@@ -181,7 +181,7 @@ struct su2gpu_pool {
   std::vector<cudaEvent_t> cyc_ev;
   // n: sweeps per replay; per_pass: one launch per pass even where the group
   // would sweep persistently
-  struct GroupGraph { int a0, a1, n; bool per_pass; cudaGraphExec_t exec; };
+  struct GroupGraph { int a0, a1, n; bool per_pass, overlap; cudaGraphExec_t exec; };
   std::vector<GroupGraph> ggraphs;
   ConvItem* h_items = nullptr;  // page-locked conversion items of a cycle (2 per chain)
   size_t h_items_n = 0;
@@ -192,8 +192,10 @@ struct su2gpu_pool {
 
 // group helpers (defined with the C entry points below)
 extern "C" {
-static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass);
-static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass);
+static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass,
+                       bool overlap = true);
+static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass,
+                               bool overlap = true);
 static std::vector<int> make_groups(const su2gpu_pool* P, int G, bool light_ends);
 static int sweep_streams(su2gpu_pool* P, int NS, std::vector<cudaStream_t>& ss);
 static int ensure_events(std::vector<cudaEvent_t>& v, size_t n);
@@ -560,7 +562,7 @@ void sweep_recipe(const su2gpu_params& p, std::vector<PassDesc>& out, int64_t* t
 // one sweep of the active chains [a0, a1) (default: all), whose tiles are the
 // tables given, one launch per pass
 int enqueue_pool_sweep(su2gpu_pool* P, const void* descs, const int2* const* tiles, const int* nt,
-                       int64_t* tot, int a0 = 0, int a1 = -1) {
+                       int64_t* tot, int a0 = 0, int a1 = -1, bool overlap = true) {
   if (a1 < 0) a1 = (int)P->active.size();
   const int* mslots = (const int*)P->mslots.p + P->h_mfirst[a0];
   const int nm = P->h_mfirst[a1] - P->h_mfirst[a0];
@@ -572,6 +574,7 @@ int enqueue_pool_sweep(su2gpu_pool* P, const void* descs, const int2* const* til
   a.descs = descs;
   a.nslots = P->max_slots;
   a.err = (int*)P->err.p;
+  a.apart = !overlap;
   for (const PassDesc& q : passes) {
     const int kind = q.kind, v = kind >= 5 ? 0 : P->var[kind];
     a.parity = q.parity; a.sub = q.sub; a.alg = q.alg; a.pass = q.pass;
@@ -1317,7 +1320,7 @@ static bool group_persistent(const su2gpu_pool* P, int a0, int a1) {
 
 // `n` sweeps of the active chains [a0, a1): their tile ranges and sweep
 // counters (persistent: one launch; otherwise one launch per pass and sweep)
-static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass) {
+static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass, bool overlap) {
   uint32_t* const* sweeps = (uint32_t* const*)P->sweepptrs.p + a0;
   if (!per_pass && group_persistent(P, a0, a1)) {
     const int4* sg = (const int4*)P->segs.p + P->h_sfirst[a0];
@@ -1331,7 +1334,7 @@ static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* t
   }
   for (int k = 0; k < n; k++) {
     int64_t t1[SU2GPU_NCOUNTERS] = {0};
-    int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot, a0, a1);
+    int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot, a0, a1, overlap);
     if (rc) return rc;
     launch_pool_next_sweep(sweeps, a1 - a0, P->st);
   }
@@ -1341,9 +1344,9 @@ static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* t
 
 // the sweep graph of the group [a0, a1) (n sweeps per replay), captured on
 // the pool's own stream
-static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass) {
+static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass, bool overlap) {
   for (auto& gg : P->ggraphs)
-    if (gg.a0 == a0 && gg.a1 == a1 && gg.n == n && gg.per_pass == per_pass) {
+    if (gg.a0 == a0 && gg.a1 == a1 && gg.n == n && gg.per_pass == per_pass && gg.overlap == overlap) {
       *out = gg.exec;
       return SU2GPU_OK;
     }
@@ -1354,7 +1357,7 @@ static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* o
   cudaGraph_t graph;
   PCK(cudaStreamBeginCapture(P->st, cudaStreamCaptureModeThreadLocal));
   int64_t tot[SU2GPU_NCOUNTERS] = {0};
-  int rc = enqueue_group_sweep(P, a0, a1, n, tot, per_pass);
+  int rc = enqueue_group_sweep(P, a0, a1, n, tot, per_pass, overlap);
   cudaError_t e = cudaStreamEndCapture(P->st, &graph);
   P->st = exec;
   if (rc) return rc;
@@ -1363,7 +1366,7 @@ static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* o
   e = cudaGraphInstantiate(&ge, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return fail(SU2GPU_ERR_CUDA, "group graph instantiate: %s", cudaGetErrorString(e));
-  P->ggraphs.push_back({a0, a1, n, per_pass, ge});
+  P->ggraphs.push_back({a0, a1, n, per_pass, overlap, ge});
   *out = ge;
   return SU2GPU_OK;
 }
@@ -1476,11 +1479,21 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
   int NS = any_persistent ? 1 : std::min(G, G <= SMALL_CYCLE_GROUPS ? SMALL_CYCLE_STREAMS : 3);
   if (const char* e = getenv("SU2GPU_CYCLE_STREAMS"); e && *e && !any_persistent)
     NS = std::max(1, std::min(std::min(G, su2gpu_pool::CYCLE_SWEEP_STREAMS), atoi(e)));
+  // Passes that start while the one before them drains take, in a cycle of many
+  // groups, room from the other streams' passes, which fill the gaps anyway:
+  // with one scalar field and no U(1) field they are launched normally.  p25 of
+  // the step in ms, normal / overlapping: 384 adjoint chains of 1.3 GB 25.8-26.4 /
+  // 27.3, half of them 13.0 / 13.4, 190 fundamental ones 12.9 / 13.4.  Elsewhere
+  // overlapping is faster: with U(1) and singlet, 0.7 of the chains, 43.2 / 38.0,
+  // doublet and triplet, half, 25.7 / 24.9; FP64 fundamental, a tenth, 42.5 / 42.2;
+  // few groups (0.08 of the adjoint chains) 2.54 / 2.43.
+  const bool one_scalar = P->content == SU2GPU_HIGGS1 || P->content == SU2GPU_TRIPLET;
+  const bool overlap = G <= SMALL_CYCLE_GROUPS || P->prec == 64 || !one_scalar;
   std::vector<cudaStream_t> ss;
   if ((rc = sweep_streams(P, NS, ss))) return rc;
   if (use_graph && nsweeps > 0)
     for (int g = 0; g < G; g++)
-      if ((rc = group_graph(P, groups[g], groups[g + 1], per_replay[g], &gex[g], false))) return rc;
+      if ((rc = group_graph(P, groups[g], groups[g + 1], per_replay[g], &gex[g], false, overlap))) return rc;
   // staging bytes of every group; a group's chains sit side by side in the
   // rings (a ring holds the largest group at least), so a chain only ever
   // overlaps chains of earlier groups, whose release events are recorded
@@ -1562,7 +1575,7 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
             for (int k = 0; k < nsweeps; k += per_replay[g]) PCK(cudaGraphLaunch(gex[g], P->st));
           } else {
             int64_t t1[SU2GPU_NCOUNTERS] = {0};
-            if (int r = enqueue_group_sweep(P, a0, a1, nsweeps, t1, false)) return r;
+            if (int r = enqueue_group_sweep(P, a0, a1, nsweeps, t1, false, overlap)) return r;
           }
         }
         if (sums) enqueue_group_measure(P, a0, a1, (double*)P->sums.p);

@@ -85,3 +85,28 @@ def test_small_cycle_groups(gpu):
         assert np.array_equal(sums[k], mb[y])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("content,precision", [("adj", 32), ("fund", 32), ("su2u1s", 32), ("fund", 64)])
+def test_cycle_of_many_groups(gpu, content, precision, graph, monkeypatch):
+    # more than 8 groups: passes launched normally (one FP32 scalar field, no
+    # U(1)) or overlapping (the others), either way the separate calls' results
+    monkeypatch.setenv("SU2GPU_CYCLE_GROUPS", "10")
+    sides = (SIDES * 3)[:13]
+    a, sa, _ = make_pool(gpu, content, precision, sides, False)
+    b, sb, fields = make_pool(gpu, content, precision, sides, None)
+    want = [{k: np.ascontiguousarray(v) for k, v in as_dict(f).items() if v is not None} for f in fields]
+    got = [{k: v.copy() for k, v in f.items()} for f in want]
+    for _ in range(2):
+        a.upload_many(sa, want)
+        a.run(2, graph=graph)
+        ma = a.measure()
+        a.download_many(sa, want)
+        mb = b.cycle(sb, got, 2, graph=graph)
+        for j, s in enumerate(sa):
+            assert np.array_equal(mb[j], ma[s])
+            assert all(np.array_equal(got[j][k], want[j][k]) for k in want[j])
+    assert all(np.array_equal(a.counters(x), b.counters(y)) for x, y in zip(sa, sb))
+    a.close()
+    b.close()
