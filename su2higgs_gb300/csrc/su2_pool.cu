@@ -1336,7 +1336,7 @@ static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* t
     int64_t t1[SU2GPU_NCOUNTERS] = {0};
     int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot, a0, a1, overlap);
     if (rc) return rc;
-    launch_pool_next_sweep(sweeps, a1 - a0, P->st);
+    launch_pool_next_sweep(sweeps, a1 - a0, P->st, 1, overlap);
   }
   PCK(cudaGetLastError());
   return SU2GPU_OK;
