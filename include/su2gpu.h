@@ -428,8 +428,10 @@ int su2gpu_pool_set_sweep(su2gpu_pool* pool, int32_t slot, uint32_t sweep);
  * pass, segment of tiles) items of all chains, each item waiting only for
  * its own chain's previous pass; use_graph != 0 replays it from a graph
  * captured for this number of sweeps.  Otherwise every pass is one launch
- * over all chains and use_graph != 0 replays one captured sweep.  Both modes
- * give the same fields bit for bit. */
+ * over all chains, or over a group of them on one of several streams, and
+ * use_graph != 0 replays captured sweeps; pools of small chains are swept in
+ * one launch with a cluster of blocks per chain.  All modes give the same
+ * fields bit for bit. */
 int su2gpu_pool_run(su2gpu_pool* pool, int32_t nsweeps, int32_t use_graph);
 /* Persistent mode: 1 on, 0 off (one launch per pass), -1 automatic (the
  * default: persistent for 8 chains or more with at least 16 tiles of 128
@@ -458,8 +460,9 @@ int su2gpu_pool_get_persist_shape(su2gpu_pool* pool, int32_t* shape, int32_t* th
  * so that the passes of several groups run side by side on the GPU.  Same
  * fields and counters as the other modes, bit for bit.  groups <= 1: off.
  * It takes precedence over the automatic persistent choice, not over a
- * forced one (su2gpu_pool_set_persistent(pool, 1)), and is not used for
- * pools with multicanonical chains.  su2gpu_pool_autotune times a few
+ * forced one (su2gpu_pool_set_persistent(pool, 1)), and an explicit choice is
+ * not used for pools with multicanonical chains.  In the automatic mode pools
+ * that neither the persistent nor the team sweep takes are grouped too.  su2gpu_pool_autotune times a few
  * (groups, streams) pairs against the pool's other mode and keeps the
  * fastest when the mode is automatic.  get: the groups and streams in
  * effect (0 and 1 when off). */

@@ -1482,7 +1482,7 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
   // Passes that start while the one before them drains take, in a cycle of many
   // groups, room from the other streams' passes, which fill the gaps anyway:
   // with one scalar field and no U(1) field they are launched normally.  p25 of
-  // the step in ms, normal / overlapping: 384 adjoint chains of 1.3 GB 25.8-26.4 /
+  // the step in ms, normal / overlapping: 384 adjoint chains of 1.3 GB 25.8-26.0 /
   // 27.3, half of them 13.0 / 13.4, 190 fundamental ones 12.9 / 13.4.  Elsewhere
   // overlapping is faster: with U(1) and singlet, 0.7 of the chains, 43.2 / 38.0,
   // doublet and triplet, half, 25.7 / 24.9; FP64 fundamental, a tenth, 42.5 / 42.2;

@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(BS, MINB) k_pool_persist(PersistArgs a) {
 // blocks, which runs all its passes of all the sweeps in one launch with a
 // cluster barrier after each pass.  A pass of a small chain is a few warps'
 // work, about 1.5 us of load and arithmetic latency; launched by itself it
-// takes 4-6 us (start, tile table, descriptor, drain), which no number of
+// takes 3-6 us (start, tile table, descriptor, drain), which no number of
 // chains hides below ~6000 warps a pass.  Here a block stages its chain's
 // descriptor once.  Block r of C takes the sites r NT, r NT + C NT, ... (NT
 // threads) of every pass.  The barrier's release and acquire order a pass's
