@@ -343,8 +343,9 @@ __device__ inline R localact_u1link(const Fields<R>& f, const Geom& g, const Cou
 // an FP32 reciprocal of the slope: the first leaves ~1e-12 of the root's
 // scale, the second rounding.  FP64 Cardano (a square root, a cube root, two
 // divisions, ~95 FP64 instructions, each holding the pipe 16 cycles) stays
-// for the cubics where that start is no good: the last correction has to be
-// below 1e-10 of the root's scale.
+// for the cubics where that start is no good: FP32 has no root of its own, the
+// slope is beyond FP32 (its reciprocal would be 0 and a correction of 0 mean
+// nothing), or the last correction is above 1e-10 of the root.
 // ---------------------------------------------------------------------------
 __device__ inline double polysolve3_f64(double a, double b, double c, double d, int* fallback);
 template <typename R>
@@ -369,13 +370,14 @@ __device__ inline R polysolve3(R a, R b, R c, R d, int* fallback) {
   }
   return x;
 }
-// one Newton step with the slope's reciprocal in FP32; the correction is returned
-__device__ inline double newton3(double a, double b, double c, double d, double* x) {
+// one Newton step with the slope's reciprocal in FP32; whether that slope is in
+// FP32's range, and the correction
+__device__ inline bool newton3(double a, double b, double c, double d, double* x, double* dx) {
   const double fx = fma(fma(fma(a, *x, b), *x, c), *x, d);
   const double dfx = fma(fma(3.0 * a, *x, 2.0 * b), *x, c);
-  const double dx = fx * (double)(1.0f / (float)dfx);
-  *x -= dx;
-  return dx;
+  *dx = fx * (double)(1.0f / (float)dfx);
+  *x -= *dx;
+  return fabs(dfx) < 1e37;
 }
 __device__ inline double polysolve3_f64(double a, double b, double c, double d, int* fallback) {
   const double discr = 18.0 * a * b * c * d - 4.0 * b * b * b * d + b * b * c * c - 4.0 * a * c * c * c - 27.0 * a * a * d * d;
@@ -384,11 +386,11 @@ __device__ inline double polysolve3_f64(double a, double b, double c, double d, 
     return b / a;
   }
   int fb = 0;
-  double x = (double)polysolve3<float>((float)a, (float)b, (float)c, (float)d, &fb);
-  newton3(a, b, c, d, &x);
-  const double dx = newton3(a, b, c, d, &x);
-  // an FP32 root of another branch, an overflow or a NaN fails this test
-  if (!(fabs(dx) <= 1e-10 * fabs(x))) {
+  double x = (double)polysolve3<float>((float)a, (float)b, (float)c, (float)d, &fb), dx;
+  newton3(a, b, c, d, &x, &dx);
+  const bool in_range = newton3(a, b, c, d, &x, &dx);
+  // an FP32 root of another branch or a NaN fails the last test
+  if (fb || !in_range || !(fabs(dx) <= 1e-10 * fabs(x))) {
     const double del1 = 2.0 * b * b * b - 9.0 * a * b * c + 27.0 * a * a * d;
     const double A = cbrt(0.5 * (del1 + a * sqrt(-27.0 * discr)));
     x = -(b + A + (b * b - 3.0 * a * c) / A) / (3.0 * a);
