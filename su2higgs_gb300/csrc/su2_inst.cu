@@ -119,9 +119,8 @@ static void l_measure(const void* f, const Geom& g, const Coup& cp, const double
                    partials);
 }
 static void l_flow(const void* fin, const void* fout, const Geom& g, const Coup& cp, double dt,
-                   unsigned long long* fz, unsigned* arrive, unsigned nb, cudaStream_t st) {
-  k_flow<R, CCI><<<nb, BLOCK, 0, st>>>(*(const Fields<R>*)fin, *(const Fields<R>*)fout, g, coup_as<R>(cp), (R)dt, fz,
-                                       arrive);
+                   unsigned long long* fz, unsigned nb, cudaStream_t st) {
+  k_flow<R, CCI><<<nb, BLOCK, 0, st>>>(*(const Fields<R>*)fin, *(const Fields<R>*)fout, g, coup_as<R>(cp), (R)dt, fz);
 }
 
 static void lp_measure(const PoolArgs& a, double* partials, unsigned nb, cudaStream_t st) {
@@ -169,6 +168,11 @@ static void p_export(const void* f, int64_t V, int kind, int h, double* dst, cud
 static void p_reunit(const void* f, int64_t V, const uint32_t* sweep, int interval, cudaStream_t st) {
   k_reunitarize<R><<<nblk(V * 3, 256), 256, 0, st>>>(*(const Fields<R>*)f, V, sweep, interval);
 }
+static void p_fixup(const void* fin, const void* fout, const Geom& g, const unsigned long long* fz,
+                    unsigned long long* next, cudaStream_t st) {
+  const unsigned nb = std::min<unsigned>(nblk((int64_t)g.V * 3, 256), FIXUP_BLOCKS);
+  launch_dependent(k_flow_fixup<R>, nb, 256, st, *(const Fields<R>*)fin, *(const Fields<R>*)fout, g, fz, next);
+}
 static void p_measure_local(const void* f, const Geom& g, const Coup& cp, double denom, double* out,
                             cudaStream_t st) {
   k_measure_local<R><<<nblk(g.V, BLOCK), BLOCK, 0, st>>>(*(const Fields<R>*)f, g, coup_as<R>(cp), denom, out);
@@ -182,7 +186,7 @@ static void p_pool_convert(const void* descs, const ConvItem* items, int n, int 
   dim3 grid(std::min(nblk(vmax, 256), 128u), (unsigned)n);
   k_pool_convert<R><<<grid, 256, 0, st>>>(descs, items, staging, to_device);
 }
-const PrecOps SU2_WITH_PREC = {p_orderparam, p_restore, p_muca_finish, p_alpha, p_import, p_export, p_reunit,
+const PrecOps SU2_WITH_PREC = {p_orderparam, p_restore, p_muca_finish, p_alpha, p_import, p_export, p_reunit, p_fixup,
                                p_measure_local, p_measure_z, p_pool_convert};
 #endif
 

@@ -23,7 +23,7 @@ struct Ops {
   void (*measure)(const void* f, const Geom& g, const Coup& cp, const double* alpha, double* partials,
                   unsigned nblocks, cudaStream_t st);
   void (*flow)(const void* fin, const void* fout, const Geom& g, const Coup& cp, double dt,
-               unsigned long long* first_zero, unsigned* arrive, unsigned nblocks, cudaStream_t st);
+               unsigned long long* first_zero, unsigned nblocks, cudaStream_t st);
   // measurement of pools of chains (su2_pool.cuh): nblocks = length of the
   // measurement tile table
   void (*pool_measure)(const PoolArgs& a, double* partials, unsigned nblocks, cudaStream_t st);
@@ -52,6 +52,10 @@ struct PrecOps {
   void (*import)(const void* f, int64_t V, int kind, int h, const double* src, cudaStream_t st);
   void (*exportf)(const void* f, int64_t V, int kind, int h, double* dst, cudaStream_t st);
   void (*reunitarize)(const void* f, int64_t V, const uint32_t* sweep, int interval, cudaStream_t st);
+  // after ops->flow: links from the first zero-force one on put back, and the
+  // next step's marker set
+  void (*flow_fixup)(const void* fin, const void* fout, const Geom& g, const unsigned long long* first_zero,
+                     unsigned long long* next_zero, cudaStream_t st);
   // per-site Tr Sigma^2 and magnetic charge / denom, out[2 V] (storage order)
   void (*measure_local)(const void* f, const Geom& g, const Coup& cp, double denom, double* out, cudaStream_t st);
   // plane sums along direction zdir: out[L[zdir]][4] (phi^2, Tr Sigma^2, S, S^2)

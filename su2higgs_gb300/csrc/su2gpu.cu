@@ -101,8 +101,8 @@ struct DevBuf {
   }
 };
 
-// device words of a context: error flag, sweep number, flow marker and arrival
-// counts, then from byte 4096 the counters (CTR_COPIES copies)
+// device words of a context: error flag, sweep number, flow markers and arrival
+// count, then from byte 4096 the counters (CTR_COPIES copies)
 constexpr size_t CTR_OFF = 4096;
 constexpr size_t CTRBUF_BYTES = CTR_OFF + CTR_BYTES;
 
@@ -1209,15 +1209,17 @@ static int flow_impl(su2gpu_ctx* c, Fields<R>& main, double t_max, double dt, in
     return SU2GPU_OK;
   };
   if ((rc = meas(t))) return rc;
-  // the first zero-force link's marker and the blocks' arrival count, which
-  // every step leaves as it found them
-  CK(cudaMemsetAsync(c->d_fz, 0xff, 8, c->st));
-  CK(cudaMemsetAsync(c->d_fz + 1, 0, 4, c->st));
+  // the markers of the first zero-force link, used in turn (flow_fixup sets the
+  // next step's)
+  CK(cudaMemsetAsync(c->d_fz, 0xff, 16, c->st));
   int iter = 1;
   unsigned nb = nblk(V, BLOCK);
   while (t < t_max) {
     if (t + dt > t_max) dt = t_max - t;
-    c->ops->flow(&A, &B, c->g, cp, dt, c->d_fz, (unsigned*)(c->d_fz + 1), nb, c->st);
+    unsigned long long* fz = c->d_fz + (iter & 1);
+    c->ops->flow(&A, &B, c->g, cp, dt, fz, nb, c->st);
+    CKL();
+    c->pops->flow_fixup(&A, &B, c->g, fz, c->d_fz + (iter + 1 & 1), c->st);
     CKL();
     std::swap(A, B);
     t += dt;
