@@ -1226,26 +1226,43 @@ static int pool_enqueue(su2gpu_pool* P, int32_t nsweeps, int32_t use_graph) {
     const int per = Gn <= 2 * NS || nsweeps % 2 ? 1 : 2;
     std::vector<cudaGraphExec_t> gex(Gn, nullptr);
     PCK(cudaEventRecord(P->grp_ev[0], P->st));
-    for (int k = 0; k < NS; k++) PCK(cudaStreamWaitEvent(ss[k], P->grp_ev[0], 0));
-    for (int g0 = 0; g0 < Gn; g0 += NS)
-      for (int k = 0; k < nsweeps; k += per)
-        for (int g = g0; g < std::min(g0 + NS, Gn); g++) {
-          if (use_graph) {
-            if (!gex[g] && (rc = group_graph(P, P->h_groups[g], P->h_groups[g + 1], per, &gex[g], true))) return rc;
-            PCK(cudaGraphLaunch(gex[g], ss[g % NS]));
-          } else {
+    // whatever fails from here on, the streams that were forked are joined
+    // below: what is already enqueued stays ordered before the pool's next call.
+    // A graph that cannot be made costs only its saving, its group's passes are
+    // then launched one by one: a run has no way back once some groups sweep.
+    auto fork = [&]() -> int {
+      for (int k = 0; k < NS; k++) PCK(cudaStreamWaitEvent(ss[k], P->grp_ev[0], 0));
+      for (int g0 = 0; g0 < Gn; g0 += NS)
+        for (int k = 0; k < nsweeps; k += per)
+          for (int g = g0; g < std::min(g0 + NS, Gn); g++) {
+            const int a0 = P->h_groups[g], a1 = P->h_groups[g + 1];
+            if (use_graph && k == 0 && group_graph(P, a0, a1, per, &gex[g], true)) {
+              gex[g] = nullptr;
+              cudaGetLastError();
+            }
+            if (gex[g]) {
+              PCK(cudaGraphLaunch(gex[g], ss[g % NS]));
+              continue;
+            }
             cudaStream_t home = P->st;
             P->st = ss[g % NS];
             int64_t t1[SU2GPU_NCOUNTERS] = {0};
-            rc = enqueue_group_sweep(P, P->h_groups[g], P->h_groups[g + 1], per, t1, true);
+            const int r = enqueue_group_sweep(P, a0, a1, per, t1, true);
             P->st = home;
-            if (rc) return rc;
+            if (r) return r;
           }
-        }
+      return SU2GPU_OK;
+    };
+    rc = fork();
+    if (rc) cudaGetLastError();  // returned here, not by the next call
+    cudaError_t je = cudaSuccess;
     for (int k = 0; k < NS; k++) {
-      PCK(cudaEventRecord(P->grp_ev[k + 1], ss[k]));
-      PCK(cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0));
+      cudaError_t e = cudaEventRecord(P->grp_ev[k + 1], ss[k]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0);
+      if (e != cudaSuccess) je = e;
     }
+    if (rc) return rc;
+    if (je != cudaSuccess) return fail(SU2GPU_ERR_CUDA, "joining the groups' streams: %s", cudaGetErrorString(je));
     std::vector<PassDesc> passes;
     sweep_recipe(P->recipe, passes, tot);
   } else if (use_graph) {
@@ -1353,14 +1370,17 @@ static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* o
   cudaStream_t exec = P->st;
   PCK(cudaStreamSynchronize(exec));
   PCK(cudaStreamSynchronize(P->own_st));
+  cudaGraph_t graph = nullptr;
+  PCK(cudaStreamBeginCapture(P->own_st, cudaStreamCaptureModeThreadLocal));
   P->st = P->own_st;
-  cudaGraph_t graph;
-  PCK(cudaStreamBeginCapture(P->st, cudaStreamCaptureModeThreadLocal));
   int64_t tot[SU2GPU_NCOUNTERS] = {0};
   int rc = enqueue_group_sweep(P, a0, a1, n, tot, per_pass, overlap);
   cudaError_t e = cudaStreamEndCapture(P->st, &graph);
   P->st = exec;
-  if (rc) return rc;
+  if (rc) {
+    if (graph) cudaGraphDestroy(graph);
+    return rc;
+  }
   if (e != cudaSuccess) return fail(SU2GPU_ERR_CUDA, "group graph capture: %s", cudaGetErrorString(e));
   cudaGraphExec_t ge;
   e = cudaGraphInstantiate(&ge, graph, 0);

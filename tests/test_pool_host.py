@@ -1,0 +1,91 @@
+"""Host code of the pool's grouped sweep, on a CUDA runtime that runs nothing
+(fake_gpu.py): what it enqueues where, and what it leaves behind when a call
+fails."""
+import pytest
+
+from fake_gpu import fake_gpu
+from su2higgs_gb300 import abi
+
+SIDES = [(16, 32, 34), (20, 24, 40), (30, 32, 28), (24, 28, 30), (26, 26, 26)]
+
+
+@pytest.fixture
+def env(monkeypatch, tmp_path_factory):
+    return fake_gpu(monkeypatch, tmp_path_factory.getbasetemp())
+
+
+def make_pool(gpu, sides=SIDES, **kw):
+    params = [abi.make_params("adj", L=L, precision=32, **kw) for L in sides]
+    pool = gpu.Pool(params[0], arena_bytes=sum(gpu.Pool.chain_bytes(p) for p in params), max_chains=len(sides))
+    for k, p in enumerate(params):
+        pool.add(p, seed=k, chain=k)
+    return pool
+
+
+def forked_and_joined(ops):
+    """(streams with work that other streams' calls wait for, streams joined):
+    a stream is forked once it waits for an event of the pool's stream and
+    joined when the pool's stream waits for an event recorded on it last."""
+    records, worked, home = {}, {}, None
+    joined = set()
+    for what, a, b in ops:
+        if what == "record":
+            home = a if home is None else home
+            records[b] = a
+        elif what in ("launch", "graph"):
+            worked[a] = True
+            joined.discard(a)
+        elif what == "wait" and a == home and b in records and records[b] != home:
+            joined.add(records[b])
+    worked.pop(home, None)
+    return set(worked), joined
+
+
+@pytest.mark.parametrize("what,n,graph", [("instantiate", 1, True), ("instantiate", 3, True), ("begin capture", 1, True),
+                                          ("end capture", 2, True), ("graph", 1, True), ("graph", 5, True),
+                                          ("launch", 40, False), ("launch", 7, False)])
+def test_a_failing_call_leaves_no_stream_unjoined(env, what, n, graph):
+    gpu, fake = env
+    pool = make_pool(gpu)
+    assert pool.sweep_groups == (4, 4)
+    fake.reset()
+    fake.fail(what, n)
+    try:
+        pool.run(2, graph=graph)
+        failed = False
+    except gpu.SU2GPUError:
+        failed = True
+    assert fake.failed(what)
+    ops = fake.ops()
+    captured = {a for w, a, _ in ops if w == "begin capture"}
+    worked, joined = forked_and_joined(ops)
+    worked -= captured  # what was launched there was captured, not run
+    assert worked and worked <= joined
+    # only launches that fail fail the run: without a graph its group's passes
+    # are launched one by one
+    assert failed == (what in ("graph", "launch"))
+    # the next run is a normal one
+    fake.reset()
+    pool.run(2, graph=graph)
+    worked, joined = forked_and_joined([o for o in fake.ops()])
+    assert len(worked - captured) == 4 and worked - captured <= joined
+    pool.close()
+
+
+def test_a_run_without_a_graph_launches_every_sweep(env):
+    gpu, fake = env
+    pool = make_pool(gpu)
+    fake.reset()
+    fake.fail("instantiate", 1)  # the second group's
+    pool.run(3)
+    ops = fake.ops()
+    captured = {a for w, a, _ in ops if w == "begin capture"}
+    passes = pool.launches_per_sweep() // 4
+    replays, launches = {}, {}
+    for w, a, _ in ops:
+        if w == "graph":
+            replays[a] = replays.get(a, 0) + 1
+        if w == "launch" and a not in captured:
+            launches[a] = launches.get(a, 0) + 1
+    assert sorted(replays.values()) == [3, 3, 3] and list(launches.values()) == [3 * passes]
+    pool.close()
