@@ -461,11 +461,12 @@ int su2gpu_pool_get_persist_shape(su2gpu_pool* pool, int32_t* shape, int32_t* th
  * fields and counters as the other modes, bit for bit.  groups <= 1: off.
  * It takes precedence over the automatic persistent choice, not over a
  * forced one (su2gpu_pool_set_persistent(pool, 1)), and an explicit choice is
- * not used for pools with multicanonical chains.  In the automatic mode pools
- * that neither the persistent nor the team sweep takes are grouped too.  su2gpu_pool_autotune times a few
- * (groups, streams) pairs against the pool's other mode and keeps the
- * fastest when the mode is automatic.  get: the groups and streams in
- * effect (0 and 1 when off). */
+ * not used for pools with multicanonical chains.  Until this is called, pools
+ * in the automatic mode that neither the persistent nor the team sweep takes
+ * are grouped too; off turns that off as well.  su2gpu_pool_autotune times a
+ * few (groups, streams) pairs against the mode the pool takes without any, and
+ * keeps the fastest when the mode is automatic.  get: the groups and streams
+ * in effect (0 and 1 when off). */
 int su2gpu_pool_set_sweep_groups(su2gpu_pool* pool, int32_t groups, int32_t streams);
 int su2gpu_pool_get_sweep_groups(su2gpu_pool* pool, int32_t* groups, int32_t* streams);
 /* Check of the persistent kernel's bounded dependency wait: runs it on a

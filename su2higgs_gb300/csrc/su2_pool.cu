@@ -172,9 +172,11 @@ struct su2gpu_pool {
   std::vector<cudaEvent_t> grp_ev;
   // the grouped sweep mode (one launch per pass, the chains split into
   // grp_G groups of about equal sites whose sweeps run on grp_NS streams in
-  // turn; grp_G <= 1: off), its groups (active-chain ranges) and whether it
+  // turn; grp_G <= 1: none chosen, and with grp_off the automatic choice may
+  // not group either), its groups (active-chain ranges) and whether it
   // is in effect for the current membership
   int grp_G = 0, grp_NS = 1;
+  bool grp_off = false;
   std::vector<int> h_groups;
   bool grouped = false;
   int run_NS = 1;  // the streams in effect: grp_NS, or the automatic choice's
@@ -344,7 +346,7 @@ int choose_teams(su2gpu_pool* P, bool fits) {
 constexpr int GROUP_STREAMS = 4;
 constexpr int64_t GROUP_BYTES = 60 << 20, ONE_ROUND_BYTES = 90 << 20;
 void choose_groups(su2gpu_pool* P) {
-  if (P->grouped || P->persistent || P->team || P->persist_mode >= 0 || P->active.size() < 2) return;
+  if (P->grp_off || P->grouped || P->persistent || P->team || P->persist_mode >= 0 || P->active.size() < 2) return;
   int64_t bytes = 0;
   for (int s : P->active) bytes += (int64_t)P->slots[s].bytes;
   if (P->prec == 64 && bytes > ONE_ROUND_BYTES) return;
@@ -1850,6 +1852,7 @@ int su2gpu_pool_set_sweep_groups(su2gpu_pool* P, int32_t groups, int32_t streams
   PCK(cudaStreamSynchronize(P->st));
   P->grp_G = groups > 1 ? groups : 0;
   P->grp_NS = groups > 1 ? streams : 1;
+  P->grp_off = groups <= 1;
   P->dirty = true;
   drop_graphs(P);
   return SU2GPU_OK;
@@ -2028,6 +2031,26 @@ int su2gpu_pool_autotune(su2gpu_pool* P, int32_t* choices, float* best_ms) {
   int rc;
   if (P->dirty && (rc = rebuild(P))) return rc;
   if (P->active.empty()) return SU2GPU_OK;
+  const char* fixg = getenv("SU2GPU_SWEEP_GROUPS");
+  if (fixg && !*fixg) fixg = nullptr;
+  // whether (groups, streams) pairs are compared below, against the mode the
+  // pool takes without any that were set or picked before; those come back if
+  // this call fails
+  const bool regroup = !fixg && P->persist_mode == -1 && P->nmuca == 0 && P->active.size() >= 8;
+  struct Before {
+    su2gpu_pool* P;
+    int G, NS;
+    ~Before() {
+      if (G <= 1) return;
+      P->grp_G = G;
+      P->grp_NS = NS;
+      P->dirty = true;
+    }
+  } before{P, regroup ? P->grp_G : 0, P->grp_NS};
+  if (before.G > 1) {
+    P->grp_G = 0;
+    if ((rc = rebuild(P))) return rc;
+  }
   size_t used = 0;
   for (int s : P->active) used = std::max(used, P->slots[s].off + P->slots[s].bytes);
   Buf arena2, slot2, desc2;
@@ -2162,15 +2185,15 @@ int su2gpu_pool_autotune(su2gpu_pool* P, int32_t* choices, float* best_ms) {
   // sweeps of every chain per candidate (groups x streams), on the scratch copy
   // SU2GPU_SWEEP_GROUPS="G,NS" fixes the pick (a profiler that serialises
   // kernels cannot time the overlap the grouped mode is for)
-  const char* fixg = getenv("SU2GPU_SWEEP_GROUPS");
-  if (!rc && fixg && *fixg) {
+  if (!rc && fixg) {
     int g = 0, ns = 1;
     if (sscanf(fixg, "%d,%d", &g, &ns) >= 1) {
       P->grp_G = g > 1 ? g : 0;
       P->grp_NS = std::max(1, std::min(ns, su2gpu_pool::CYCLE_SWEEP_STREAMS));
+      P->grp_off = g <= 1;
       P->dirty = true;
     }
-  } else if (!rc && P->persist_mode == -1 && P->nmuca == 0 && P->active.size() >= 8) {
+  } else if (!rc && regroup) {
     const int na = (int)P->active.size();
     if (P->team) {
       float ms = 0.f;
@@ -2187,9 +2210,9 @@ int su2gpu_pool_autotune(su2gpu_pool* P, int32_t* choices, float* best_ms) {
       if (!rc) base_ms = ms / reps / TUNE_SWEEPS;
     }
     // the automatic choice's groups, or one launch per pass
-    const bool own = P->grouped && P->grp_G <= 1;
     if (!rc && base_ms <= 0.f &&
-        (rc = time_grouped(P, desc2.p, own ? (int)P->h_groups.size() - 1 : 1, own ? P->run_NS : 1, reps, &base_ms))) {
+        (rc = time_grouped(P, desc2.p, P->grouped ? (int)P->h_groups.size() - 1 : 1, P->grouped ? P->run_NS : 1, reps,
+                           &base_ms))) {
       // base_ms stays unset; rc is returned below
     }
     // (groups, streams): on the 384-chain ensemble (11 M sites) groups of
@@ -2223,8 +2246,10 @@ int su2gpu_pool_autotune(su2gpu_pool* P, int32_t* choices, float* best_ms) {
     // the mode the pool would use anyway
     if (bg && !(bestg < 0.98f * base_ms)) bg = 0;
     if (!rc) {
+      before.G = 0;
       P->grp_G = bg;
       P->grp_NS = bg ? bns : 1;
+      if (bg) P->grp_off = false;
       P->dirty = true;
     }
   }

@@ -652,7 +652,8 @@ class Pool:
 
     @sweep_groups.setter
     def sweep_groups(self, gs):
-        """(groups, streams); None or groups <= 1: off."""
+        """(groups, streams); None or groups <= 1: off, the automatic choice's
+        groups too."""
         g, n = (0, 1) if gs is None else gs
         check(lib().su2gpu_pool_set_sweep_groups(self._h, int(g), int(n)))
 

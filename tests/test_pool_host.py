@@ -89,3 +89,62 @@ def test_a_run_without_a_graph_launches_every_sweep(env):
             launches[a] = launches.get(a, 0) + 1
     assert sorted(replays.values()) == [3, 3, 3] and list(launches.values()) == [3 * passes]
     pool.close()
+
+
+def test_groups_off_is_off(env):
+    gpu, fake = env
+    pool = make_pool(gpu)
+    assert pool.sweep_groups == (4, 4)  # the automatic choice
+    for off in (None, (1, 3), (0, 1), (-1, 1)):
+        pool.sweep_groups = (3, 2)
+        assert pool.sweep_groups == (3, 2)
+        pool.sweep_groups = off
+        assert pool.sweep_groups == (0, 1)
+        fake.reset()
+        pool.run(2)
+        assert len({a for w, a, _ in fake.ops() if w == "graph"}) == 1
+    # off does not depend on the other mode, and stays until it is set again
+    pool.persistent = False
+    pool.persistent = None
+    assert pool.sweep_groups == (0, 1)
+    pool.sweep_groups = (2, 2)
+    assert pool.sweep_groups == (2, 2)
+    pool.close()
+
+
+def test_autotuner_with_groups_fixed_off(env, monkeypatch):
+    gpu, fake = env
+    pool = make_pool(gpu, SIDES * 2)
+    monkeypatch.setenv("SU2GPU_SWEEP_GROUPS", "1,1")
+    pool.autotune()
+    assert pool.sweep_groups == (0, 1)
+    pool.close()
+
+
+def test_autotuner_again_compares_with_the_automatic_choice(env):
+    gpu, fake = env
+
+    def captures(groups):
+        pool = make_pool(gpu, SIDES * 2)
+        if groups:
+            pool.sweep_groups = groups
+        fake.reset()
+        pool.autotune()  # every launch takes the same time: nothing is picked
+        n = sum(w == "begin capture" for w, _, _ in fake.ops())
+        left = pool.sweep_groups
+        pool.close()
+        return n, left
+
+    assert captures((5, 3)) == captures(None)
+
+
+def test_failed_autotuner_leaves_the_groups(env):
+    gpu, fake = env
+    pool = make_pool(gpu, SIDES * 2)
+    pool.sweep_groups = (5, 3)
+    fake.reset()
+    fake.fail("instantiate", 6)
+    with pytest.raises(gpu.SU2GPUError):
+        pool.autotune()
+    assert fake.failed("instantiate") and pool.sweep_groups == (5, 3)
+    pool.close()
