@@ -231,12 +231,17 @@ int su2gpu_device_info(int* sm_count, int* cc_major, int* cc_minor, int64_t* fre
   return SU2GPU_OK;
 }
 
+// a context's partial sums: of an update's or a measurement's blocks
+static size_t partials_bytes(int64_t V) {
+  return (size_t)(std::max(nblk(V, BLOCK), meas_blocks((int)V)) + 2) * NSUMS * 8;
+}
+
 int64_t su2gpu_footprint_bytes(const su2gpu_params* p) {
   if (!valid_params(p)) return -1;
   int64_t V = (int64_t)p->L[0] * p->L[1] * p->L[2];
   size_t b = field_bytes(p, V);
-  b += align256((size_t)(V / BLOCK + 2) * NSUMS * 8);        // partials
-  b += 4096;                                                 // counters, flags, sums
+  b += align256(partials_bytes(V));
+  b += align256(CTRBUF_BYTES) + align256(NSUMS * 8);         // counters, flags, sums
   if (p->content & SU2GPU_TRIPLET) b += align256(3 * V * 8);  // alpha planes
   return (int64_t)b;
 }
@@ -271,7 +276,7 @@ static int create_ctx(const su2gpu_params* p, void* borrowed, const void* copy_f
   }
   if ((!borrowed && (rc = c->fields.ensure(field_bytes(p, V)))) ||
       (rc = c->ctrbuf.ensure(CTRBUF_BYTES)) ||
-      (rc = c->partials.ensure((size_t)(std::max(nblk(V, BLOCK), meas_blocks((int)V)) + 2) * NSUMS * 8)) ||
+      (rc = c->partials.ensure(partials_bytes(V))) ||
       (rc = c->sums.ensure(NSUMS * 8))) {
     su2gpu_destroy(c);
     return rc;
