@@ -1932,7 +1932,9 @@ static int pool_enqueue_measure(su2gpu_pool* P, double* dev_out, int32_t max_cha
 
 int su2gpu_pool_measure(su2gpu_pool* P, double* sums, int32_t max_chains, int32_t* nchains) {
   if (!P || !sums || !nchains) return SU2GPU_ERR_INVALID;
-  int rc = pool_enqueue_measure(P, (double*)P->sums.p, max_chains, nchains);
+  int rc;
+  if (P->dirty && (rc = rebuild(P))) return rc;  // the sums' buffer is sized there
+  rc = pool_enqueue_measure(P, (double*)P->sums.p, max_chains, nchains);
   if (rc || !*nchains) return rc;
   PCK(cudaMemcpyAsync(sums, P->sums.p, (size_t)*nchains * NSUMS * 8, cudaMemcpyDeviceToHost, P->st));
   PCK(cudaStreamSynchronize(P->st));

@@ -26,10 +26,22 @@ cudaError_t last = cudaSuccess;
 std::set<cudaStream_t> capturing;
 int64_t numbers = 0;
 float elapsed = 1.0f;
+std::map<const void*, std::string> names;  // kernels by the address of their host stub
+std::string watched;
+int watched_arg = 0;
+uint64_t watched_value = 0;
+
+cudaError_t step(const char* what, const void* a = nullptr, const void* b = nullptr);
+cudaError_t launch(const void* f, void** args, cudaStream_t st) {
+  auto n = names.find(f);
+  if (!watched.empty() && n != names.end() && n->second.find(watched) != std::string::npos)
+    memcpy(&watched_value, args[watched_arg], 8);
+  return step("launch", st);
+}
 
 int64_t id(const void* p) { return (int64_t)(intptr_t)p; }
 void* handle() { return (void*)(intptr_t)++numbers; }
-cudaError_t step(const char* what, const void* a = nullptr, const void* b = nullptr) {
+cudaError_t step(const char* what, const void* a, const void* b) {
   auto f = fail_after.find(what);
   if (f != fail_after.end() && f->second-- == 0) {
     fail_after.erase(f);
@@ -44,11 +56,22 @@ cudaError_t step(const char* what, const void* a = nullptr, const void* b = null
 
 extern "C" {
 // ---- the test's side
-void fake_reset() { ops.clear(); fail_after.clear(); elapsed = 1.0f; last = cudaSuccess; }
+void fake_reset() { ops.clear(); fail_after.clear(); elapsed = 1.0f; last = cudaSuccess; watched.clear(); }
 void fake_fail(const char* what, int n) { fail_after[what] = n; }
 int fake_failed(const char* what) { return !fail_after.count(what); }
 void fake_elapsed(float ms) { elapsed = ms; }
 int64_t fake_live_bytes() { return live; }
+// the 8 bytes of argument `arg` of the kernel whose name holds `name`, at its last launch
+void fake_watch(const char* name, int arg) { watched = name; watched_arg = arg; watched_value = 0; }
+uint64_t fake_watched() { return watched_value; }
+// bytes from p to the end of the allocation that holds it (0: none does)
+int64_t fake_room(uint64_t p) {
+  for (auto& b : blocks) {
+    const uint64_t lo = (uint64_t)(uintptr_t)b.first;
+    if (p >= lo && p < lo + b.second) return (int64_t)(lo + b.second - p);
+  }
+  return 0;
+}
 int fake_ops() { return (int)ops.size(); }
 const char* fake_op(int k, int64_t* a, int64_t* b) { *a = ops[k].a; *b = ops[k].b; return ops[k].what; }
 
@@ -56,17 +79,19 @@ const char* fake_op(int k, int64_t* a, int64_t* b) { *a = ops[k].a; *b = ops[k].
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
-void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
+  names[f] = name;
+}
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 static thread_local cudaStream_t pushed;
 unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, cudaStream_t st) { pushed = st; return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void* st) { *(cudaStream_t*)st = pushed; return cudaSuccess; }
 cudaError_t __cudaGetKernel(void** k, const void* f) { *k = (void*)f; return cudaSuccess; }
-cudaError_t __cudaLaunchKernel(void*, dim3, dim3, void**, size_t, cudaStream_t st) { return step("launch", st); }
+cudaError_t __cudaLaunchKernel(void* k, dim3, dim3, void** args, size_t, cudaStream_t st) { return launch(k, args, st); }
 
 // ---- the runtime
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*, void**) { return step("launch", c->stream); }
-cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t st) { return step("launch", st); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) { return launch(f, args, c->stream); }
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t st) { return launch(f, args, st); }
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no error" : "fake error"; }
 cudaError_t cudaMalloc(void** p, size_t n) {

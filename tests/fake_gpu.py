@@ -28,6 +28,9 @@ class Fake:
         lib.fake_op.restype = ctypes.c_char_p
         lib.fake_live_bytes.restype = ctypes.c_int64
         lib.fake_elapsed.argtypes = [ctypes.c_float]
+        lib.fake_watched.restype = ctypes.c_uint64
+        lib.fake_room.restype = ctypes.c_int64
+        lib.fake_room.argtypes = [ctypes.c_uint64]
 
     def reset(self):
         self.lib.fake_reset()
@@ -41,6 +44,14 @@ class Fake:
 
     def live_bytes(self):
         return self.lib.fake_live_bytes()
+
+    def watch(self, kernel, arg):
+        """Keep argument `arg` (8 bytes) of the kernel's next launches."""
+        self.lib.fake_watch(kernel.encode(), arg)
+
+    def room(self):
+        """Bytes of device memory from the watched pointer on."""
+        return self.lib.fake_room(self.lib.fake_watched())
 
     def ops(self):
         a, b = ctypes.c_int64(), ctypes.c_int64()
