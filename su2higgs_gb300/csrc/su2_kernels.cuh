@@ -2220,7 +2220,11 @@ __device__ inline void flow_site(const Fields<R>& in, const Fields<R>& out, cons
     }
     // flow_gauge (gradflow.c:361-401)
     if (mod <= (R)0) {
-      atomicMin(first_zero, (unsigned long long)(i * 3 + mu));
+      // one atomic a warp, and none above the marker: a start without forces
+      // otherwise sends 3 V of them to one address, 0.5 ms a step at 64^3
+      const unsigned k = (unsigned)(i * 3 + mu);
+      if (k == __reduce_min_sync(__activemask(), k) && k < *(volatile unsigned long long*)first_zero)
+        atomicMin(first_zero, (unsigned long long)k);
       st4<R>(lk(out, mu), i, U);
       continue;
     }
@@ -2265,9 +2269,11 @@ __global__ void __launch_bounds__(BLOCK) k_flow(Fields<R> in, Fields<R> out, Geo
 // (the reference's early return in flow_gauge), and the other of the two markers
 // is made ready for the next step.  A launch over the whole GPU, since a start
 // with no gauge force at all (unit links, no triplet) keeps every link in every
-// step: 64^3, 10 steps with measurements, 0.53 ms; with the step's last block
-// putting them back by itself 24 ms.  Without a zero force it only looks at the
-// marker, most of that under the step's end.
+// step: 64^3, 10 steps with measurements, 0.27 ms; with the step's last block
+// putting them back by itself 20 ms.  Without a zero force it only looks at the
+// marker, most of that under the step's end (64^3, 20 steps: 581 us for the whole
+// flow, 606 with the step's blocks counting themselves in, 728 with a launch
+// before and one after each step).
 constexpr int FIXUP_BLOCKS = 152 * 8;
 template <typename R>
 __global__ void __launch_bounds__(256) k_flow_fixup(Fields<R> in, Fields<R> out, Geom g,
