@@ -1202,14 +1202,14 @@ __global__ void __launch_bounds__(128) k_link_split(Fields<double> f, PassArgs a
     R d = (s_log[0][lane] * s_cos[lane] + s_log[1][lane]) * ia;
     R r3 = 1.0 - draw_at(rng, 3);
     int trials = 1;
-    bool ok = r3 * r3 <= 1.0 - 0.5 * d;
+    bool ok = !(r3 * r3 > 1.0 - 0.5 * d);  // a NaN ends the trials, as in heatbath
     while (!ok && trials < 200) {
       const uint32_t n = 4u * (uint32_t)trials;
       const R u0 = draw_at(rng, n), u1 = rng.uni(), cs = mcos2pi(rng.uni());
       r3 = 1.0 - rng.uni();
       d = (-log(1.0 - u0) * (cs * cs) - log(1.0 - u1)) * ia;
       trials++;
-      ok = r3 * r3 <= 1.0 - 0.5 * d;
+      ok = !(r3 * r3 > 1.0 - 0.5 * d);
     }
     R a0 = 1.0 - d;
     if (trials >= 200) {  // the loop's cap, even if the last trial succeeded
@@ -1217,7 +1217,7 @@ __global__ void __launch_bounds__(128) k_link_split(Fields<double> f, PassArgs a
       cap = 1;
     }
     R rad = 1.0 - a0 * a0;
-    if (rad >= 0.0) {
+    if (!(rad < 0.0)) {
       rad = sqrt(rad);
       R n1 = s_n[0][lane], n2 = s_n[1][lane], n3 = s_n[2][lane];
       int nd = s_nd[lane];
