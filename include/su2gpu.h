@@ -463,7 +463,8 @@ int su2gpu_pool_get_persist_shape(su2gpu_pool* pool, int32_t* shape, int32_t* th
  * forced one (su2gpu_pool_set_persistent(pool, 1)), and an explicit choice is
  * not used for pools with multicanonical chains.  Until this is called, pools
  * in the automatic mode that neither the persistent nor the team sweep takes
- * are grouped too; off turns that off as well.  su2gpu_pool_autotune times a
+ * are grouped too (FP32 pools of less than 400,000 sites only where graphs are
+ * replayed); off turns that off as well.  su2gpu_pool_autotune times a
  * few (groups, streams) pairs against the mode the pool takes without any, and
  * keeps the fastest when the mode is automatic.  get: the groups and streams
  * in effect (0 and 1 when off). */

@@ -179,6 +179,7 @@ struct su2gpu_pool {
   bool grp_off = false;
   std::vector<int> h_groups;
   bool grouped = false;
+  bool direct_groups = true;  // without a graph too
   int run_NS = 1;  // the streams in effect: grp_NS, or the automatic choice's
   std::vector<cudaEvent_t> cyc_ev;
   // n: sweeps per replay; per_pass: one launch per pass even where the group
@@ -343,6 +344,16 @@ int choose_teams(su2gpu_pool* P, bool fits) {
 // 39 MB 1709 / 1307 (1306), 20 of 28 MB 1452 / 1084 (1069); of 157 MB in one
 // round 6583, in rounds of 105 MB 6019.  FP64 pools, bound by the FP64 pipe, gain
 // the gaps alone (10 chains 1289 / 1044), so only pools of one round are grouped.
+//
+// Without a graph every pass of every group is a launch by the host, ~2.3 us
+// each, and the automatic choice's groups of a small FP32 pool take longer to
+// launch than to run.  Groups against one launch per pass, us for a run of 1 / 4
+// sweeps: 0.14 M sites (10 x 24^3 adjoint) 152 / 446 against 82 / 266, 0.26 M
+// 160 / 460 against 104 / 358, 0.39 M 168 / 473 against 139 / 496, 0.44 M 176 /
+// 489 against 151 / 542, 0.66 M 193 / 588 against 192 / 708; the other contents
+// and chains with weights cross over there too.  FP64 passes are long enough at
+// every size (0.05 M sites 453 / 1616 against 467 / 1808).
+constexpr int64_t DIRECT_GROUP_SITES = 400000;
 constexpr int GROUP_STREAMS = 4;
 constexpr int64_t GROUP_BYTES = 60 << 20, ONE_ROUND_BYTES = 90 << 20;
 void choose_groups(su2gpu_pool* P) {
@@ -359,6 +370,9 @@ void choose_groups(su2gpu_pool* P) {
   }
   P->grouped = true;
   P->run_NS = std::min(G, GROUP_STREAMS);
+  int64_t sites = 0;
+  for (int s : P->active) sites += P->slots[s].g.V;
+  P->direct_groups = P->prec == 64 || sites >= DIRECT_GROUP_SITES;
 }
 
 // descriptors and tile tables for the current membership
@@ -445,6 +459,7 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
     // takes precedence over the automatic choice, not over a forced one
     P->grouped = P->grp_G > 1 && (int)P->active.size() > 1 && P->persist_mode != 1 && P->nmuca == 0;
     P->run_NS = P->grp_NS;
+    P->direct_groups = true;
     P->h_groups.clear();
     if (P->grouped) {
       P->persistent = false;
@@ -1212,7 +1227,7 @@ static int pool_enqueue(su2gpu_pool* P, int32_t nsweeps, int32_t use_graph) {
     }
   } else if (P->team) {
     if ((rc = enqueue_teams(P, sweeps, na, nsweeps, tot))) return rc;
-  } else if (P->grouped) {
+  } else if (P->grouped && (use_graph || P->direct_groups)) {
     // the groups' sweeps on run_NS streams in turn, forked from and joined
     // back into the pool's stream
     const int Gn = (int)P->h_groups.size() - 1;

@@ -15,7 +15,7 @@ def env(monkeypatch, tmp_path_factory):
 
 
 def make_pool(gpu, sides=SIDES, **kw):
-    params = [abi.make_params("adj", L=L, precision=32, **kw) for L in sides]
+    params = [abi.make_params("adj", L=L, **{"precision": 32, **kw}) for L in sides]
     pool = gpu.Pool(params[0], arena_bytes=sum(gpu.Pool.chain_bytes(p) for p in params), max_chains=len(sides))
     for k, p in enumerate(params):
         pool.add(p, seed=k, chain=k)
@@ -46,7 +46,7 @@ def forked_and_joined(ops):
                                           ("launch", 40, False), ("launch", 7, False)])
 def test_a_failing_call_leaves_no_stream_unjoined(env, what, n, graph):
     gpu, fake = env
-    pool = make_pool(gpu)
+    pool = make_pool(gpu, SIDES if graph else SIDES * 4)
     assert pool.sweep_groups == (4, 4)
     fake.reset()
     fake.fail(what, n)
@@ -147,4 +147,24 @@ def test_failed_autotuner_leaves_the_groups(env):
     with pytest.raises(gpu.SU2GPUError):
         pool.autotune()
     assert fake.failed("instantiate") and pool.sweep_groups == (5, 3)
+    pool.close()
+
+
+def streams_launched_on(fake, pool, graph):
+    fake.reset()
+    pool.run(1, graph=graph)
+    captured = {a for w, a, _ in fake.ops() if w == "begin capture"}
+    return len({a for w, a, _ in fake.ops() if w == "graph" or (w == "launch" and a not in captured)})
+
+
+@pytest.mark.parametrize("precision,copies,direct", [(32, 1, 1), (32, 3, 1), (32, 4, 4), (64, 1, 4)])
+def test_direct_launches_of_small_pools_are_not_grouped(env, precision, copies, direct):
+    # 0.1 M sites a copy; a pool's groups run side by side from 0.4 M on, FP64
+    # ones always
+    gpu, fake = env
+    pool = make_pool(gpu, SIDES * copies, precision=precision)
+    assert pool.sweep_groups == (4, 4)
+    assert streams_launched_on(fake, pool, False) == direct
+    pool.sweep_groups = (3, 2)  # what the caller asks for holds either way
+    assert streams_launched_on(fake, pool, False) == 2
     pool.close()
