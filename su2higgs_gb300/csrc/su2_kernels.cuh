@@ -510,8 +510,8 @@ __device__ inline int heatbath(const Fields<R>& f, const Geom& g, const CoupT<R>
 }
 
 // FP32 form: every link written is re-normalised to unit length, so rounding
-// never accumulates in the SU(2) constraint (the FP64 path writes the
-// reference's arithmetic unchanged)
+// never accumulates in the SU(2) constraint (the FP64 path writes the product
+// as it is, as the reference does)
 template <typename R>
 __device__ inline Q<R> unitize(const Q<R>& q) {
   if (sizeof(R) == 8) return q;
@@ -734,15 +734,12 @@ __device__ inline int overrelax_doublet(const Fields<R>& f, const Geom& g, const
   Q<R> s = staple_doublet<R, CC>(f, g, cp, c, i, 0);
   Q<R> p = ld4<R>(php(f, 0), i);
   R F = msqrt(s.a * s.a + s.b * s.b + s.c * s.c + s.d * s.d);
-  // FP32: one reciprocal instead of nine divisions (the FP64 path divides as
-  // the reference does)
-  const bool f32 = sizeof(R) == 4;
-  const R iF = f32 ? (R)1 / F : (R)0;
-  R X = f32 ? (p.a * s.a + p.b * s.b + p.c * s.c + p.d * s.d) * iF : (p.a * s.a + p.b * s.b + p.c * s.c + p.d * s.d) / F;
-  R y0 = f32 ? p.a - X * s.a * iF : p.a - X * s.a / F;
-  R y1 = f32 ? p.b - X * s.b * iF : p.b - X * s.b / F;
-  R y2 = f32 ? p.c - X * s.c * iF : p.c - X * s.c / F;
-  R y3 = f32 ? p.d - X * s.d * iF : p.d - X * s.d / F;
+  const R iF = (R)1 / F;  // one reciprocal instead of nine divisions
+  R X = (p.a * s.a + p.b * s.b + p.c * s.c + p.d * s.d) * iF;
+  R y0 = p.a - X * s.a * iF;
+  R y1 = p.b - X * s.b * iF;
+  R y2 = p.c - X * s.c * iF;
+  R y3 = p.d - X * s.d * iF;
   R Ysq = y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3;
   R B = (R)0.5 * (R)cp.msq + (R)3;
   if (HAS(C_T)) B += (R)0.5 * (R)cp.a2 * tripletsq(ld3(f, i));
@@ -757,8 +754,7 @@ __device__ inline int overrelax_doublet(const Fields<R>& f, const Geom& g, const
   R dVn = F + (R)2 * B * newX + (R)4 * C * (newX * newX * newX + Ysq * newX);
   if (mabs(dV / dVn) >= u) {
     R k = (newX + X);
-    st4<R>(php(f, 0), i, f32 ? Q<R>{-p.a + k * s.a * iF, -p.b + k * s.b * iF, -p.c + k * s.c * iF, -p.d + k * s.d * iF}
-                             : Q<R>{-p.a + k * s.a / F, -p.b + k * s.b / F, -p.c + k * s.c / F, -p.d + k * s.d / F});
+    st4<R>(php(f, 0), i, Q<R>{-p.a + k * s.a * iF, -p.b + k * s.b * iF, -p.c + k * s.c * iF, -p.d + k * s.d * iF});
     return 1;
   }
   return 0;
@@ -863,14 +859,11 @@ __device__ inline int overrelax_triplet(const Fields<R>& f, const Geom& g, const
   V3<R> s = staple_triplet(f, g, c, i);
   V3<R> t = ld3(f, i);
   R F = msqrt(s.x * s.x + s.y * s.y + s.z * s.z);
-  // FP32: one reciprocal instead of seven divisions (the FP64 path divides as
-  // the reference does)
-  const bool f32 = sizeof(R) == 4;
-  const R iF = f32 ? (R)1 / F : (R)0;
-  R X = f32 ? (t.x * s.x + t.y * s.y + t.z * s.z) * iF : (t.x * s.x + t.y * s.y + t.z * s.z) / F;
-  R y0 = f32 ? t.x - X * s.x * iF : t.x - X * s.x / F;
-  R y1 = f32 ? t.y - X * s.y * iF : t.y - X * s.y / F;
-  R y2 = f32 ? t.z - X * s.z * iF : t.z - X * s.z / F;
+  const R iF = (R)1 / F;  // one reciprocal instead of seven divisions
+  R X = (t.x * s.x + t.y * s.y + t.z * s.z) * iF;
+  R y0 = t.x - X * s.x * iF;
+  R y1 = t.y - X * s.y * iF;
+  R y2 = t.z - X * s.z * iF;
   R Ysq = y0 * y0 + y1 * y1 + y2 * y2;
   R B = (R)0.5 * (R)cp.msqT + (R)3;
   R C = (R)0.25 * (R)cp.b4;
@@ -880,8 +873,7 @@ __device__ inline int overrelax_triplet(const Fields<R>& f, const Geom& g, const
   R dVn = F + (R)2 * B * newX + (R)4 * C * (newX * newX * newX + Ysq * newX);
   if (mabs(dV / dVn) >= u) {
     R k = newX + X;
-    st3(f, i, f32 ? V3<R>{-t.x + k * s.x * iF, -t.y + k * s.y * iF, -t.z + k * s.z * iF}
-                  : V3<R>{-t.x + k * s.x / F, -t.y + k * s.y / F, -t.z + k * s.z / F});
+    st3(f, i, V3<R>{-t.x + k * s.x * iF, -t.y + k * s.y * iF, -t.z + k * s.z * iF});
     return 1;
   }
   return 0;
@@ -897,9 +889,9 @@ __device__ inline int metro_triplet(const Fields<R>& f, const Geom& g, const Cou
                                     SiteRng<R>& rng) {
   if constexpr (sizeof(R) == 8) return metro_triplet_f64<CC>(f, cp, i, staple_triplet(f, g, c, i), rng);
   const R e0 = rng.uni() - (R)0.5, e1 = rng.uni() - (R)0.5, e2 = rng.uni() - (R)0.5;
-  // FP32: the decision's uniform is the fourth word of the same generator
-  // block, drawn with the proposal; FP64 draws it only when it is needed
-  const R ua = sizeof(R) == 4 ? rng.uni() : (R)0;
+  // the decision's uniform is the fourth word of the same generator block,
+  // drawn with the proposal (FP64 draws it only when it is needed)
+  const R ua = rng.uni();
   V3<R> s = staple_triplet(f, g, c, i);
   V3<R> old = ld3(f, i);
   V3<R> nw = old;
@@ -912,7 +904,7 @@ __device__ inline int metro_triplet(const Fields<R>& f, const Geom& g, const Cou
   R B = (R)0.5 * (R)cp.msqT + (R)3;
   if (NHIGGS > 0) B += (R)0.5 * (R)cp.a2 * doubletsq(ld4<R>(php(f, 0), i));
   const R dS = dx * s.x + dy * s.y + dz * s.z + dsq * (B + (R)0.25 * (R)cp.b4 * ssq);
-  if (sizeof(R) == 4 ? metro_accept_u(dS, ua) : metro_accept(dS, rng)) {
+  if (metro_accept_u(dS, ua)) {
     st3(f, i, nw);
     return 1;
   }
