@@ -2099,24 +2099,21 @@ __device__ inline double warp_sums(const double (&v)[N]) {
 }
 
 // sums of m[] over the block (blockDim.x a multiple of 32, at most BLOCK) to
-// partials[k * nblocks + block].  The runtime content sums one value after
-// another, skipping those that its fields do not have.
+// partials[k * nblocks + block].  The runtime content sums all NSUMS values
+// (those that its fields do not have are 0 and are left out below): one tree per
+// value that it has takes longer from seven values on.
 template <int CC>
 __device__ inline void block_sums_out(const double* m, int content, double* partials, int nblocks, int block) {
   constexpr int NA = nactive_sums<CC>();
-  constexpr int N = CC == C_GENERIC ? NSUMS : (NA <= 4 ? 4 : (NA <= 8 ? 8 : (NA <= 16 ? 16 : 32)));
+  constexpr int N = CC == C_GENERIC ? 32 : (NA <= 4 ? 4 : (NA <= 8 ? 8 : (NA <= 16 ? 16 : 32)));
   __shared__ double sm[BLOCK / 32][N];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int j = -1;  // this thread's sum: its place in sm[w]
   if constexpr (CC == C_GENERIC) {
+    double v[N];
 #pragma unroll
-    for (int k = 0; k < NSUMS; k++) {
-      if (!sum_active(k, content)) continue;
-      double v = m[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) sm[w][k] = v;
-    }
+    for (int q = 0; q < N; q++) v[q] = q < NSUMS ? m[q < NSUMS ? q : 0] : 0.0;
+    sm[w][lane] = warp_sums<N, 16>(v);
     if (threadIdx.x < NSUMS && sum_active(threadIdx.x, content)) j = threadIdx.x;
   } else {
     double v[N];
@@ -2139,22 +2136,29 @@ __device__ inline void block_sums_out(const double* m, int content, double* part
 
 // Sites per thread of a measurement of V sites: up to MEAS_SPT, which spreads
 // the block's sum over many sites, but no more than leaves about eight warps per
-// SM (the sum depends on the number, so it is a function of the chain's own
-// volume alone).  With 8 everywhere a 16^3 lattice was 4 blocks.
+// SM (the sum depends on the number, so it is a function of the lattice's own
+// volume and precision alone).  With 8 everywhere a 16^3 lattice was 4 blocks.
+// FP64, where an SM quarter's warps run one after another: rounded up, so that no
+// quarter gets a third warp (64^3 fundamental: 142 us rounded down to 6 sites a
+// thread, 115 in 7, 132 in 8).
 constexpr int MEAS_SPT = 8;
-__host__ __device__ inline int meas_spt(int V) {
-  const int s = V / (32 * 8 * 152);
+__host__ __device__ inline int meas_spt(int V, bool f64) {
+  constexpr int W = 32 * 8 * 152;
+  const int s = f64 && V > 2 * W ? (V + W - 1) / W : V / W;
   return s < 1 ? 1 : (s > MEAS_SPT ? MEAS_SPT : s);
 }
 // threads per block: one warp where blocks of BLOCK would leave SMs idle
 __host__ __device__ inline int meas_threads(int V) { return V <= 2 * 152 * BLOCK ? 32 : BLOCK; }
-inline unsigned meas_blocks(int V) {
-  const int per = meas_spt(V) * meas_threads(V);
+inline unsigned meas_blocks(int V, bool f64) {
+  const int per = meas_spt(V, f64) * meas_threads(V);
   return (unsigned)((V + per - 1) / per);
 }
 
 // measure() over the whole lattice; alpha = the k_alpha planes (triplet
-// content) or null.  meas_blocks(V) blocks of meas_threads(V) threads.
+// content) or null.  meas_blocks(V) blocks of meas_threads(V) threads.  The
+// runtime content takes its full 8 sites in a loop of that many turns: with the
+// number in a register the same loop ran at 178 instead of 118 us for two doublets
+// at 96^3, 514 instead of 269 at 128^3.
 template <typename R, int CC>
 __global__ void __launch_bounds__(BLOCK) k_measure(Fields<R> f, Geom g, CoupT<R> cp, const double* alpha,
                                                    double* partials) {
@@ -2163,10 +2167,17 @@ __global__ void __launch_bounds__(BLOCK) k_measure(Fields<R> f, Geom g, CoupT<R>
 #pragma unroll
   for (int k = 0; k < NSUMS; k++) m[k] = 0.0;
   const AlphaPlanes ap{alpha, g.V};
-  const int spt = meas_spt(g.V);
-  for (int j = 0; j < spt; j++) {
-    int t = ((int)blockIdx.x * spt + j) * (int)blockDim.x + threadIdx.x;
-    if (t < g.V) measure_site<R, CC>(f, g, cp, t, ap, m);
+  const int spt = meas_spt(g.V, sizeof(R) == 8);
+  if (CC == C_GENERIC && spt == MEAS_SPT) {
+    for (int j = 0; j < MEAS_SPT; j++) {
+      int t = ((int)blockIdx.x * MEAS_SPT + j) * BLOCK + threadIdx.x;
+      if (t < g.V) measure_site<R, CC>(f, g, cp, t, ap, m);
+    }
+  } else {
+    for (int j = 0; j < spt; j++) {
+      int t = ((int)blockIdx.x * spt + j) * (int)blockDim.x + threadIdx.x;
+      if (t < g.V) measure_site<R, CC>(f, g, cp, t, ap, m);
+    }
   }
   block_sums_out<CC>(m, cp.content, partials, gridDim.x, blockIdx.x);
 }

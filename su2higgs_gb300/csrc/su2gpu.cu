@@ -232,15 +232,15 @@ int su2gpu_device_info(int* sm_count, int* cc_major, int* cc_minor, int64_t* fre
 }
 
 // a context's partial sums: of an update's or a measurement's blocks
-static size_t partials_bytes(int64_t V) {
-  return (size_t)(std::max(nblk(V, BLOCK), meas_blocks((int)V)) + 2) * NSUMS * 8;
+static size_t partials_bytes(int64_t V, int prec) {
+  return (size_t)(std::max(nblk(V, BLOCK), meas_blocks((int)V, prec == 64)) + 2) * NSUMS * 8;
 }
 
 int64_t su2gpu_footprint_bytes(const su2gpu_params* p) {
   if (!valid_params(p)) return -1;
   int64_t V = (int64_t)p->L[0] * p->L[1] * p->L[2];
   size_t b = field_bytes(p, V);
-  b += align256(partials_bytes(V));
+  b += align256(partials_bytes(V, p->precision));
   b += align256(CTRBUF_BYTES) + align256(NSUMS * 8);         // counters, flags, sums
   if (p->content & SU2GPU_TRIPLET) b += align256(3 * V * 8);  // alpha planes
   return (int64_t)b;
@@ -276,7 +276,7 @@ static int create_ctx(const su2gpu_params* p, void* borrowed, const void* copy_f
   }
   if ((!borrowed && (rc = c->fields.ensure(field_bytes(p, V)))) ||
       (rc = c->ctrbuf.ensure(CTRBUF_BYTES)) ||
-      (rc = c->partials.ensure(partials_bytes(V))) ||
+      (rc = c->partials.ensure(partials_bytes(V, p->precision))) ||
       (rc = c->sums.ensure(NSUMS * 8))) {
     su2gpu_destroy(c);
     return rc;
@@ -1011,7 +1011,7 @@ static int enqueue_measure(su2gpu_ctx* c, const void* F, const Coup& cp, double*
     c->pops->alpha(F, c->g, cp, (double*)c->alpha.p, c->st);
     CKL();
   }
-  const unsigned nb = meas_blocks((int)V);
+  const unsigned nb = meas_blocks((int)V, c->prec == 64);
   c->ops->measure(F, c->g, cp, (const double*)c->alpha.p, (double*)c->partials.p, nb, c->st);
   CKL();
   launch_reduce_partials((const double*)c->partials.p, (int)nb, out, c->st);
