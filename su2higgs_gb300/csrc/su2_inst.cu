@@ -205,8 +205,8 @@ void launch_pool_reduce(const double* partials, int nblocks, const int* first, i
                         cudaStream_t st) {
   if (nchains) k_pool_reduce<<<nchains, 32 * NSUMS, 0, st>>>(partials, nblocks, first, base, out);
 }
-void launch_pool_next_sweep(uint32_t* const* sweeps, int n, cudaStream_t st, uint32_t inc, bool overlap) {
-  if (n) launch_pass(overlap, k_pool_next_sweep, (n + 255) / 256, 256, st, sweeps, n, inc);
+void launch_pool_next_sweep(uint32_t* const* sweeps, int n, cudaStream_t st, uint32_t inc) {
+  if (n) launch_dependent(k_pool_next_sweep, (n + 255) / 256, 256, st, sweeps, n, inc);
 }
 #endif
 

@@ -23,9 +23,8 @@ namespace su2 {
 __device__ inline void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ inline void dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// overlap false: launched normally
 template <typename... P, typename... A>
-inline void launch_pass(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -34,13 +33,8 @@ inline void launch_pass(bool overlap, void (*kernel)(P...), dim3 grid, dim3 bloc
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = overlap ? 1 : 0;
+  cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-
-template <typename... P, typename... A>
-inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A&&... args) {
-  launch_pass(true, kernel, grid, block, st, static_cast<A&&>(args)...);
 }
 
 }  // namespace su2

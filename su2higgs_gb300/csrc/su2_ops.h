@@ -88,7 +88,7 @@ void launch_muca_set_param(MucaDev* w, const double* partials, int np, double vo
 void launch_reduce_partials(const double* partials, int np, double* out, cudaStream_t st);
 void launch_pool_reduce(const double* partials, int nblocks, const int* first, int base, int nchains, double* out,
                         cudaStream_t st);
-void launch_pool_next_sweep(uint32_t* const* sweeps, int n, cudaStream_t st, uint32_t inc = 1, bool overlap = true);
+void launch_pool_next_sweep(uint32_t* const* sweeps, int n, cudaStream_t st, uint32_t inc = 1);
 
 // the update kernels of pools of one (precision, content) instantiation
 // (su2_persist.cu).  launch: the persistent sweep, the work list of `args`

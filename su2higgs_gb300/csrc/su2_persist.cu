@@ -23,25 +23,25 @@ template <int V>
 static void lp_link_v(const PoolArgs& a, unsigned nb, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
   if (!nb) return;
-  if (a.sub == 0) launch_pass(!a.apart, k_pool_link<R, CCI, 0, BS, MB>, nb, BS, st, a);
-  else if (a.sub == 1) launch_pass(!a.apart, k_pool_link<R, CCI, 1, BS, MB>, nb, BS, st, a);
-  else launch_pass(!a.apart, k_pool_link<R, CCI, 2, BS, MB>, nb, BS, st, a);
+  if (a.sub == 0) launch_dependent(k_pool_link<R, CCI, 0, BS, MB>, nb, BS, st, a);
+  else if (a.sub == 1) launch_dependent(k_pool_link<R, CCI, 1, BS, MB>, nb, BS, st, a);
+  else launch_dependent(k_pool_link<R, CCI, 2, BS, MB>, nb, BS, st, a);
 }
 template <int V>
 static void lp_u1_v(const PoolArgs& a, unsigned nb, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
   if (!nb) return;
-  if (a.sub == 0) launch_pass(!a.apart, k_pool_u1<R, CCI, 0, BS, MB>, nb, BS, st, a);
-  else if (a.sub == 1) launch_pass(!a.apart, k_pool_u1<R, CCI, 1, BS, MB>, nb, BS, st, a);
-  else launch_pass(!a.apart, k_pool_u1<R, CCI, 2, BS, MB>, nb, BS, st, a);
+  if (a.sub == 0) launch_dependent(k_pool_u1<R, CCI, 0, BS, MB>, nb, BS, st, a);
+  else if (a.sub == 1) launch_dependent(k_pool_u1<R, CCI, 1, BS, MB>, nb, BS, st, a);
+  else launch_dependent(k_pool_u1<R, CCI, 2, BS, MB>, nb, BS, st, a);
 }
 template <int V>
 static void lp_scalar_v(int field, const PoolArgs& a, unsigned nb, cudaStream_t st) {
   constexpr int BS = Variant<R, V>::BS, MB = Variant<R, V>::MINB;
   if (!nb) return;
-  if (field == 0) launch_pass(!a.apart, k_pool_scalar<R, CCI, 0, BS, MB>, nb, BS, st, a);
-  else if (field == 1) launch_pass(!a.apart, k_pool_scalar<R, CCI, 1, BS, MB>, nb, BS, st, a);
-  else launch_pass(!a.apart, k_pool_scalar<R, CCI, 2, BS, MB>, nb, BS, st, a);
+  if (field == 0) launch_dependent(k_pool_scalar<R, CCI, 0, BS, MB>, nb, BS, st, a);
+  else if (field == 1) launch_dependent(k_pool_scalar<R, CCI, 1, BS, MB>, nb, BS, st, a);
+  else launch_dependent(k_pool_scalar<R, CCI, 2, BS, MB>, nb, BS, st, a);
 }
 static void lp_link(int v, const PoolArgs& a, unsigned nb, cudaStream_t st) {
   switch (v) {

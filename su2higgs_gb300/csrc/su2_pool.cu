@@ -164,6 +164,7 @@ struct su2gpu_pool {
   // the download copy stream, and one sweep graph per group of chains
   Buf ring_down;
   cudaStream_t down_st = nullptr;
+  cudaStream_t copy_hi = nullptr, down_hi = nullptr;  // both at the sweeps' priority
   // update streams of the grouped sweep and the cycle, forked from and
   // joined back into st: the sweeps of consecutive groups run side by side
   // (highest priority, as own_st, whatever the caller's stream)
@@ -184,7 +185,7 @@ struct su2gpu_pool {
   std::vector<cudaEvent_t> cyc_ev;
   // n: sweeps per replay; per_pass: one launch per pass even where the group
   // would sweep persistently
-  struct GroupGraph { int a0, a1, n; bool per_pass, overlap; cudaGraphExec_t exec; };
+  struct GroupGraph { int a0, a1, n; bool per_pass; cudaGraphExec_t exec; };
   std::vector<GroupGraph> ggraphs;
   ConvItem* h_items = nullptr;  // page-locked conversion items of a cycle (2 per chain)
   size_t h_items_n = 0;
@@ -195,10 +196,8 @@ struct su2gpu_pool {
 
 // group helpers (defined with the C entry points below)
 extern "C" {
-static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass,
-                       bool overlap = true);
-static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass,
-                               bool overlap = true);
+static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass);
+static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass);
 static std::vector<int> make_groups(const su2gpu_pool* P, int G, bool light_ends);
 static int sweep_streams(su2gpu_pool* P, int NS, std::vector<cudaStream_t>& ss);
 static int ensure_events(std::vector<cudaEvent_t>& v, size_t n);
@@ -580,7 +579,7 @@ void sweep_recipe(const su2gpu_params& p, std::vector<PassDesc>& out, int64_t* t
 // one sweep of the active chains [a0, a1) (default: all), whose tiles are the
 // tables given, one launch per pass
 int enqueue_pool_sweep(su2gpu_pool* P, const void* descs, const int2* const* tiles, const int* nt,
-                       int64_t* tot, int a0 = 0, int a1 = -1, bool overlap = true) {
+                       int64_t* tot, int a0 = 0, int a1 = -1) {
   if (a1 < 0) a1 = (int)P->active.size();
   const int* mslots = (const int*)P->mslots.p + P->h_mfirst[a0];
   const int nm = P->h_mfirst[a1] - P->h_mfirst[a0];
@@ -592,7 +591,6 @@ int enqueue_pool_sweep(su2gpu_pool* P, const void* descs, const int2* const* til
   a.descs = descs;
   a.nslots = P->max_slots;
   a.err = (int*)P->err.p;
-  a.apart = !overlap;
   for (const PassDesc& q : passes) {
     const int kind = q.kind, v = kind >= 5 ? 0 : P->var[kind];
     a.parity = q.parity; a.sub = q.sub; a.alg = q.alg; a.pass = q.pass;
@@ -729,8 +727,6 @@ int su2gpu_pool_create(const su2gpu_params* recipe, int64_t arena_bytes, int32_t
   P->max_slots = max_chains;
   P->slots.resize(max_chains);
   int rc;
-  // the update stream at the highest priority: the transfer streams' kernels
-  // (field conversions) fill in around the sweeps instead of displacing them
   int least = 0, greatest = 0;
   cudaDeviceGetStreamPriorityRange(&least, &greatest);
   if (cudaStreamCreateWithPriority(&P->own_st, cudaStreamNonBlocking, greatest) != cudaSuccess) {
@@ -786,8 +782,8 @@ int su2gpu_pool_destroy(su2gpu_pool* P) {
   for (int v = 0; v < NVARIANTS; v++) P->tiles[v].release();
   for (int k = 0; k < 2; k++)
     if (P->stage_ev[k]) cudaEventDestroy(P->stage_ev[k]);
-  if (P->copy_st) cudaStreamSynchronize(P->copy_st);
-  if (P->down_st) cudaStreamSynchronize(P->down_st);
+  for (cudaStream_t st : {P->copy_st, P->down_st, P->copy_hi, P->down_hi})
+    if (st) cudaStreamSynchronize(st);
   for (cudaStream_t x : P->sweep_st)
     if (x) cudaStreamSynchronize(x);
   P->ring.release();
@@ -797,8 +793,8 @@ int su2gpu_pool_destroy(su2gpu_pool* P) {
   for (cudaEvent_t e : P->grp_ev) cudaEventDestroy(e);
   if (P->h_items) cudaFreeHost(P->h_items);
   P->d_items.release();
-  if (P->copy_st) cudaStreamDestroy(P->copy_st);
-  if (P->down_st) cudaStreamDestroy(P->down_st);
+  for (cudaStream_t st : {P->copy_st, P->down_st, P->copy_hi, P->down_hi})
+    if (st) cudaStreamDestroy(st);
   for (cudaStream_t x : P->sweep_st)
     if (x) cudaStreamDestroy(x);
   if (P->own_st) cudaStreamDestroy(P->own_st);
@@ -1097,11 +1093,12 @@ static int ensure_events(std::vector<cudaEvent_t>& v, size_t n) {
   return SU2GPU_OK;
 }
 
-// a transfer stream, at the lowest priority
-static int ensure_stream(cudaStream_t* st) {
+// a transfer stream; conversions on it fill in around the sweeps, or
+// (before_sweeps) take turns with them
+static int ensure_stream(cudaStream_t* st, bool before_sweeps = false) {
   int least = 0, greatest = 0;
   cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  if (!*st && cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, least) != cudaSuccess)
+  if (!*st && cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, before_sweeps ? greatest : least) != cudaSuccess)
     return fail(SU2GPU_ERR_CUDA, "cudaStreamCreate failed");
   return SU2GPU_OK;
 }
@@ -1111,8 +1108,8 @@ static int ensure_stream(cudaStream_t* st) {
 static int ensure_ring(su2gpu_pool* P, Buf& buf, size_t total, size_t largest, Ring* R) {
   const size_t want = std::max(largest, std::min(total, ring_bytes()));
   if (buf.n < want) {
-    if (P->copy_st) PCK(cudaStreamSynchronize(P->copy_st));
-    if (P->down_st) PCK(cudaStreamSynchronize(P->down_st));
+    for (cudaStream_t st : {P->copy_st, P->down_st, P->copy_hi, P->down_hi})
+      if (st) PCK(cudaStreamSynchronize(st));
     PCK(cudaStreamSynchronize(P->st));
     int rc = buf.ensure(want);
     if (rc) return rc;
@@ -1355,7 +1352,7 @@ static bool group_persistent(const su2gpu_pool* P, int a0, int a1) {
 
 // `n` sweeps of the active chains [a0, a1): their tile ranges and sweep
 // counters (persistent: one launch; otherwise one launch per pass and sweep)
-static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass, bool overlap) {
+static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* tot, bool per_pass) {
   uint32_t* const* sweeps = (uint32_t* const*)P->sweepptrs.p + a0;
   if (!per_pass && group_persistent(P, a0, a1)) {
     const int4* sg = (const int4*)P->segs.p + P->h_sfirst[a0];
@@ -1369,9 +1366,9 @@ static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* t
   }
   for (int k = 0; k < n; k++) {
     int64_t t1[SU2GPU_NCOUNTERS] = {0};
-    int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot, a0, a1, overlap);
+    int rc = enqueue_pool_sweep(P, P->descs.p, tiles, nt, k ? t1 : tot, a0, a1);
     if (rc) return rc;
-    launch_pool_next_sweep(sweeps, a1 - a0, P->st, 1, overlap);
+    launch_pool_next_sweep(sweeps, a1 - a0, P->st);
   }
   PCK(cudaGetLastError());
   return SU2GPU_OK;
@@ -1379,9 +1376,9 @@ static int enqueue_group_sweep(su2gpu_pool* P, int a0, int a1, int n, int64_t* t
 
 // the sweep graph of the group [a0, a1) (n sweeps per replay), captured on
 // the pool's own stream
-static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass, bool overlap) {
+static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* out, bool per_pass) {
   for (auto& gg : P->ggraphs)
-    if (gg.a0 == a0 && gg.a1 == a1 && gg.n == n && gg.per_pass == per_pass && gg.overlap == overlap) {
+    if (gg.a0 == a0 && gg.a1 == a1 && gg.n == n && gg.per_pass == per_pass) {
       *out = gg.exec;
       return SU2GPU_OK;
     }
@@ -1392,7 +1389,7 @@ static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* o
   PCK(cudaStreamBeginCapture(P->own_st, cudaStreamCaptureModeThreadLocal));
   P->st = P->own_st;
   int64_t tot[SU2GPU_NCOUNTERS] = {0};
-  int rc = enqueue_group_sweep(P, a0, a1, n, tot, per_pass, overlap);
+  int rc = enqueue_group_sweep(P, a0, a1, n, tot, per_pass);
   cudaError_t e = cudaStreamEndCapture(P->st, &graph);
   P->st = exec;
   if (rc) {
@@ -1404,7 +1401,7 @@ static int group_graph(su2gpu_pool* P, int a0, int a1, int n, cudaGraphExec_t* o
   e = cudaGraphInstantiate(&ge, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return fail(SU2GPU_ERR_CUDA, "group graph instantiate: %s", cudaGetErrorString(e));
-  P->ggraphs.push_back({a0, a1, n, per_pass, overlap, ge});
+  P->ggraphs.push_back({a0, a1, n, per_pass, ge});
   *out = ge;
   return SU2GPU_OK;
 }
@@ -1450,12 +1447,23 @@ static std::vector<int> make_groups(const su2gpu_pool* P, int G, bool light_ends
 // 8 of 20 MB on up to six streams instead, so that the transfers of most groups
 // and the gaps between most passes are covered (64 chains, 141 MB: 2 groups 2490
 // us, 4 on 4 streams 2325, 6 on 6 2180, 8 on 6 2160, 16 on 6 2590).
+//
+// The field conversions of few groups, on streams of the lowest priority, fill in
+// around their sweeps; those of many take turns with the sweeps, at their
+// priority.  There, passes that start while the one before them drains always have
+// blocks waiting for room, and a conversion of lower priority waits for all of
+// them, and with it the groups whose upload or download it is.  ms a step, lowest /
+// the sweeps' priority: six streams, adjoint, 3 groups of 64 MB 2.88 / 2.85, 6
+// groups 5.6 / 6.0, doublet + triplet, 5 groups 7.7 / 8.8; three streams, adjoint, 9
+// groups 7.9 / 7.7, 12 9.35 / 9.1, 35 27.4 / 24.8 (25.9 at the lowest with the passes
+// launched normally), SU(2)xU(1) + singlet, 5 sweeps, 25 groups 20.1 / 18.3.
 constexpr int SMALL_CYCLE_GROUPS = 8, SMALL_CYCLE_STREAMS = 6;
+constexpr int64_t CYCLE_GROUP_BYTES = 64 << 20;
 static std::vector<int> cycle_groups(const su2gpu_pool* P) {
   int64_t total = 0;
   for (int s : P->active) total += P->slots[s].g.V;
   const int64_t bytes = total * STAGE_REALS * 8;
-  int G = (int)std::min<int64_t>(32, bytes / (64ll << 20));
+  int G = (int)std::min<int64_t>(32, bytes / CYCLE_GROUP_BYTES);
   if (G < SMALL_CYCLE_GROUPS) G = (int)std::min<int64_t>(SMALL_CYCLE_GROUPS, std::max<int64_t>(1, bytes / (20ll << 20)));
   const char* e = getenv("SU2GPU_CYCLE_GROUPS");
   if (e && *e) G = std::max(1, atoi(e));
@@ -1514,24 +1522,16 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
   // blocks, each pass with its ramp and tail) run on NS streams in turn, so
   // that consecutive groups fill each other's gaps; persistent groups share
   // the work counters and stay on one stream
-  int NS = any_persistent ? 1 : std::min(G, G <= SMALL_CYCLE_GROUPS ? SMALL_CYCLE_STREAMS : 3);
+  const bool many = G > SMALL_CYCLE_GROUPS || total >= (size_t)SMALL_CYCLE_GROUPS * CYCLE_GROUP_BYTES;
+  int NS = any_persistent ? 1 : std::min(G, many ? 3 : SMALL_CYCLE_STREAMS);
   if (const char* e = getenv("SU2GPU_CYCLE_STREAMS"); e && *e && !any_persistent)
     NS = std::max(1, std::min(std::min(G, su2gpu_pool::CYCLE_SWEEP_STREAMS), atoi(e)));
-  // Passes that start while the one before them drains take, in a cycle of many
-  // groups, room from the other streams' passes, which fill the gaps anyway:
-  // with one scalar field and no U(1) field they are launched normally.  p25 of
-  // the step in ms, normal / overlapping: 384 adjoint chains of 1.3 GB 25.8-26.0 /
-  // 27.3, half of them 13.0 / 13.4, 190 fundamental ones 12.9 / 13.4.  Elsewhere
-  // overlapping is faster: with U(1) and singlet, 0.7 of the chains, 43.2 / 38.0,
-  // doublet and triplet, half, 25.7 / 24.9; FP64 fundamental, a tenth, 42.5 / 42.2;
-  // few groups (0.08 of the adjoint chains) 2.54 / 2.43.
-  const bool one_scalar = P->content == SU2GPU_HIGGS1 || P->content == SU2GPU_TRIPLET;
-  const bool overlap = G <= SMALL_CYCLE_GROUPS || P->prec == 64 || !one_scalar;
+  cudaStream_t &copy = many ? P->copy_hi : P->copy_st, &down_copy = many ? P->down_hi : P->down_st;
   std::vector<cudaStream_t> ss;
   if ((rc = sweep_streams(P, NS, ss))) return rc;
   if (use_graph && nsweeps > 0)
     for (int g = 0; g < G; g++)
-      if ((rc = group_graph(P, groups[g], groups[g + 1], per_replay[g], &gex[g], false, overlap))) return rc;
+      if ((rc = group_graph(P, groups[g], groups[g + 1], per_replay[g], &gex[g], false))) return rc;
   // staging bytes of every group; a group's chains sit side by side in the
   // rings (a ring holds the largest group at least), so a chain only ever
   // overlaps chains of earlier groups, whose release events are recorded
@@ -1540,7 +1540,7 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
     for (int a = groups[g]; a < groups[g + 1]; a++) gbytes[g] += (size_t)P->slots[P->active[a]].g.V * STAGE_REALS * 8;
   const size_t gmax = *std::max_element(gbytes.begin(), gbytes.end());
   Ring up, down;
-  if ((rc = ensure_stream(&P->copy_st)) || (rc = ensure_stream(&P->down_st)) ||
+  if ((rc = ensure_stream(&copy, many)) || (rc = ensure_stream(&down_copy, many)) ||
       (rc = ensure_ring(P, P->ring, total, gmax, &up)) || (rc = ensure_ring(P, P->ring_down, total, gmax, &down)) ||
       (rc = ensure_events(P->cyc_ev, 4 * (size_t)G + 1 + NS)) || (rc = P->d_items.ensure(2 * (size_t)na * sizeof(ConvItem))))
     return rc;
@@ -1555,8 +1555,8 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
   ConvItem* dit = (ConvItem*)P->d_items.p;
   // the fields may still be in use by earlier work on st
   PCK(cudaEventRecord(ev[4 * G], P->st));
-  PCK(cudaStreamWaitEvent(P->copy_st, ev[4 * G], 0));
-  PCK(cudaStreamWaitEvent(P->down_st, ev[4 * G], 0));
+  PCK(cudaStreamWaitEvent(copy, ev[4 * G], 0));
+  PCK(cudaStreamWaitEvent(down_copy, ev[4 * G], 0));
   for (int k = 0; k < NS; k++) PCK(cudaStreamWaitEvent(ss[k], ev[4 * G], 0));
   int64_t tot[SU2GPU_NCOUNTERS] = {0};
   // one chain's host arrays and their staging layout
@@ -1589,18 +1589,18 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
       size_t bytes, lo;
       ConvItem& it = P->h_items[a];
       const ChainIo io = layout(a, in, hp, &it, &bytes);
-      if ((rc = ring_take(up, bytes, P->copy_st, &lo))) return rc;
+      if ((rc = ring_take(up, bytes, copy, &lo))) return rc;
       it.off = (long long)(lo / 8);
       size_t off = 0;
       for (int k = 0; k < io.count; k++) {
-        PCK(cudaMemcpyAsync((double*)(up.base + lo) + off, hp[k], io.n[k] * 8, cudaMemcpyHostToDevice, P->copy_st));
+        PCK(cudaMemcpyAsync((double*)(up.base + lo) + off, hp[k], io.n[k] * 8, cudaMemcpyHostToDevice, copy));
         off += io.n[k];
       }
       up.live.push_back({lo, lo + bytes, ev[4 * g + 1]});
     }
-    PCK(cudaMemcpyAsync(dit + a0, P->h_items + a0, (a1 - a0) * sizeof(ConvItem), cudaMemcpyHostToDevice, P->copy_st));
-    P->pops->pool_convert(P->descs.p, dit + a0, a1 - a0, vmax, (double*)up.base, 1, P->copy_st);
-    PCK(cudaEventRecord(ev[4 * g + 1], P->copy_st));
+    PCK(cudaMemcpyAsync(dit + a0, P->h_items + a0, (a1 - a0) * sizeof(ConvItem), cudaMemcpyHostToDevice, copy));
+    P->pops->pool_convert(P->descs.p, dit + a0, a1 - a0, vmax, (double*)up.base, 1, copy);
+    PCK(cudaEventRecord(ev[4 * g + 1], copy));
     // update stream of the group: its sweeps and measurement (the enqueue
     // helpers launch on P->st, pointed at that stream meanwhile)
     {
@@ -1613,7 +1613,7 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
             for (int k = 0; k < nsweeps; k += per_replay[g]) PCK(cudaGraphLaunch(gex[g], P->st));
           } else {
             int64_t t1[SU2GPU_NCOUNTERS] = {0};
-            if (int r = enqueue_group_sweep(P, a0, a1, nsweeps, t1, false, overlap)) return r;
+            if (int r = enqueue_group_sweep(P, a0, a1, nsweeps, t1, false)) return r;
           }
         }
         if (sums) enqueue_group_measure(P, a0, a1, (double*)P->sums.p);
@@ -1626,7 +1626,7 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
     }
     // download stream: one conversion launch into staging, then the copies
     // to the host arrays
-    PCK(cudaStreamWaitEvent(P->down_st, ev[4 * g + 2], 0));
+    PCK(cudaStreamWaitEvent(down_copy, ev[4 * g + 2], 0));
     std::vector<std::pair<ChainIo, size_t>> outs;
     std::vector<std::array<double*, 6>> outp;
     for (int a = a0; a < a1; a++) {
@@ -1634,25 +1634,25 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
       size_t bytes, lo;
       ConvItem& it = P->h_items[na + a];
       const ChainIo io = layout(a, out, hp.data(), &it, &bytes);
-      if ((rc = ring_take(down, bytes, P->down_st, &lo))) return rc;
+      if ((rc = ring_take(down, bytes, down_copy, &lo))) return rc;
       it.off = (long long)(lo / 8);
       outs.push_back({io, lo});
       outp.push_back(hp);
       down.live.push_back({lo, lo + bytes, ev[4 * g + 3]});
     }
     PCK(cudaMemcpyAsync(dit + na + a0, P->h_items + na + a0, (a1 - a0) * sizeof(ConvItem), cudaMemcpyHostToDevice,
-                        P->down_st));
-    P->pops->pool_convert(P->descs.p, dit + na + a0, a1 - a0, vmax, (double*)down.base, 0, P->down_st);
+                        down_copy));
+    P->pops->pool_convert(P->descs.p, dit + na + a0, a1 - a0, vmax, (double*)down.base, 0, down_copy);
     for (size_t q = 0; q < outs.size(); q++) {
       const ChainIo& io = outs[q].first;
       size_t off = 0;
       for (int k = 0; k < io.count; k++) {
         PCK(cudaMemcpyAsync(outp[q][k], (double*)(down.base + outs[q].second) + off, io.n[k] * 8,
-                            cudaMemcpyDeviceToHost, P->down_st));
+                            cudaMemcpyDeviceToHost, down_copy));
         off += io.n[k];
       }
     }
-    PCK(cudaEventRecord(ev[4 * g + 3], P->down_st));
+    PCK(cudaEventRecord(ev[4 * g + 3], down_copy));
     PCK(cudaGetLastError());
   }
   // half-sweeps of each kind in one sweep of a chain
@@ -1670,8 +1670,8 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
     hs.resize((size_t)na * NSUMS);
     PCK(cudaMemcpyAsync(hs.data(), P->sums.p, hs.size() * 8, cudaMemcpyDeviceToHost, P->st));
   }
-  PCK(cudaStreamSynchronize(P->copy_st));
-  PCK(cudaStreamSynchronize(P->down_st));
+  PCK(cudaStreamSynchronize(copy));
+  PCK(cudaStreamSynchronize(down_copy));
   if ((rc = pool_check(P))) return rc;
   if (sums)
     for (int a = 0; a < na; a++) memcpy(sums + (size_t)pos[a] * NSUMS, hs.data() + (size_t)a * NSUMS, NSUMS * 8);

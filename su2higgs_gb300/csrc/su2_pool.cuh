@@ -107,7 +107,6 @@ struct PoolArgs {
   int parity, sub, alg;
   uint32_t pass;
   int* err;
-  int apart;  // host: the pass starts when the one before it has ended (launch_pass)
 };
 
 // a tile whose slot lies outside the descriptor table (a corrupted table)

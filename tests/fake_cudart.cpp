@@ -153,7 +153,10 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t*) { *n = 8; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)handle(); return cudaSuccess; }
-cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned, int) { *s = (cudaStream_t)handle(); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithPriority(cudaStream_t* s, unsigned, int priority) {
+  *s = (cudaStream_t)handle();
+  return step("stream", *s, (void*)(intptr_t)priority);
+}
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) { return step("sync", st); }
 cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t e, unsigned) { return step("wait", st, e); }

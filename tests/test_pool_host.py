@@ -1,6 +1,7 @@
 """Host code of the pool's grouped sweep, on a CUDA runtime that runs nothing
 (fake_gpu.py): what it enqueues where, and what it leaves behind when a call
 fails."""
+import numpy as np
 import pytest
 
 from fake_gpu import fake_gpu
@@ -167,4 +168,23 @@ def test_direct_launches_of_small_pools_are_not_grouped(env, precision, copies, 
     assert streams_launched_on(fake, pool, False) == direct
     pool.sweep_groups = (3, 2)  # what the caller asks for holds either way
     assert streams_launched_on(fake, pool, False) == 2
+    pool.close()
+
+
+@pytest.mark.parametrize("groups,turns", [(4, False), (10, True)])
+def test_conversions_of_a_large_cycle_do_not_wait_behind_the_sweeps(env, monkeypatch, groups, turns):
+    # the sweeps' passes always have blocks waiting for room: a transfer stream
+    # of lower priority gets none until the sweeps of the groups in flight end
+    gpu, fake = env
+    monkeypatch.setenv("SU2GPU_CYCLE_GROUPS", str(groups))
+    sides = [(4, 6, 8)] * 15
+    pool = make_pool(gpu, sides)
+    fields = [{"link": np.zeros((192, 3, 4)), "trip": np.zeros((192, 3))} for _ in sides]
+    pool.cycle(list(pool.active()), fields, 2)
+    priority = {a: b for w, a, b in fake.ops() if w == "stream"}
+    swept = {a for w, a, _ in fake.ops() if w == "graph"}
+    moved = {a for w, a, _ in fake.ops() if w == "copy"} & set(priority) - swept
+    moved = {a for a in moved if sum(w == "copy" and x == a for w, x, _ in fake.ops()) >= len(sides)}
+    assert swept and len(moved) == 2  # upload and download streams
+    assert (max(priority[a] for a in moved) <= min(priority[a] for a in swept)) == turns  # less is higher
     pool.close()
