@@ -12,6 +12,9 @@ namespace su2 {
 // field content bits (same values as SU2GPU_* in include/su2gpu.h)
 // ---------------------------------------------------------------------------
 enum : int { C_H1 = 0x01, C_H2 = 0x02, C_T = 0x04, C_S = 0x08, C_U1 = 0x10 };
+// GB300's streaming multiprocessors.  Launch shapes are made for this number, and
+// not for the device's, as the order of the sums follows from them.
+constexpr int SMS = 152;
 constexpr int C_GENERIC = -1;  // content read from the runtime mask
 enum : int { ALG_METRO = 1, ALG_HEATBATH = 2, ALG_OR = 3 };
 

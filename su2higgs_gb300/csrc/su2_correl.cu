@@ -347,7 +347,7 @@ void launch_block(const PlainLat& s, const PlainLat& b, const int* bd, int has_t
 // in all, as there the chunks' sums weigh more than an even last wave
 int correl_chunks(const PlainLat& p, int dir) {
   const int Lz = p.L[dir], area = p.V / Lz;
-  const int warps = (area + 31) / 32, per = std::max(1, (int)((int64_t)warps * Lz / (152 * 64)));
+  const int warps = (area + 31) / 32, per = std::max(1, (int)((int64_t)warps * Lz / (SMS * 64)));
   return (warps + per - 1) / per;
 }
 

@@ -25,7 +25,7 @@ constexpr int CCI = SU2_CC;
 // their SM's L1: blocks of one warp cost 2-5 % there at every size tried
 // (42 x 12 x 30 to 88 x 72 x 14).
 static unsigned launch_threads(int n, int bs) {
-  if (sizeof(R) == 4 || (n + 31) / 32 > 152 * 16) return (unsigned)bs;
+  if (sizeof(R) == 4 || (n + 31) / 32 > SMS * 16) return (unsigned)bs;
   return (unsigned)std::min(bs, 32);
 }
 

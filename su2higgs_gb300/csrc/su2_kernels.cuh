@@ -342,7 +342,7 @@ __device__ inline R localact_u1link(const Fields<R>& f, const Geom& g, const Cou
 // the accuracy, the start comes from the FP32 root, and the steps multiply by
 // an FP32 reciprocal of the slope: the first leaves ~1e-12 of the root's
 // scale, the second rounding.  FP64 Cardano (a square root, a cube root, two
-// divisions, ~95 FP64 instructions, each holding the pipe 16 cycles) stays
+// divisions, ~95 FP64 instructions, each holding a quarter's pipe 64 cycles) stays
 // for the cubics where that start is no good: FP32 has no root of its own, the
 // slope is beyond FP32 (its reciprocal would be 0 and a correction of 0 mean
 // nothing), or the last correction is above 1e-10 of the root.
@@ -1103,8 +1103,10 @@ __global__ void __launch_bounds__(BS, MINB) k_scalar(Fields<R> f, PassArgs a) {
 // quarters (608) lasts as long as one site's FP64 instructions.  Each warp takes
 // a part of the staple (and of the random numbers' functions); the first goes on
 // with the sum.  Sweep + measurement of the fundamental theory, one lane a site
-// against four: 16^3 (64 groups of 32 sites) 261 / 213 us, 32^3 (512 groups, where
-// the quarters are nearly full) 299 / 306 us; the line lies between.
+// against four: 16^3 (64 groups of 32 sites) 261 / 213 us.  Two sweeps, us, over the
+// groups of 32 sites: fundamental 319 468 / 452, 352 462 / 460, 384 468 / 472, 416
+// 467 / 476, 512 482 / 525; adjoint 384 513 / 507, 416 513 / 515; SU(2)xU(1) +
+// singlet 384 833 / 812, 448 836 / 832, 480 872 / 914: the line is at 384.
 // ---------------------------------------------------------------------------
 constexpr int SPLIT_GROUPS = 384;
 
@@ -1671,8 +1673,9 @@ __device__ inline bool last_to_arrive(unsigned* arrive, unsigned n) {
 // half goes back from the backup; the block that arrives last, when all have
 // read the weight, commits the decision.  Deciding inside the update -- a fence
 // and two levels of arrivals in every one of its blocks -- made the 96^3 doublet
-// half-sweep 35 us instead of 27 us, with a restore launch still to follow.
-constexpr int MUCA_FINISH_BLOCKS = 152;
+// half-sweep 35 us, with a restore launch of 3.4 to follow; it takes 23 without,
+// and this launch 11.
+constexpr int MUCA_FINISH_BLOCKS = SMS;
 template <typename R, int FIELD>
 __global__ void __launch_bounds__(256) k_muca_finish(Fields<R> f, MucaDev* w, const double* partials, int np,
                                                      double vol, int parity, RngKey rk, uint32_t pass, uint32_t check,
@@ -2077,8 +2080,8 @@ constexpr int active_sum(int j) {
 // Sums of N (a power of two <= 32) values over the warp, each lane left with
 // one of them: at every step a lane keeps half of its values, adding the other
 // lane's, and hands the other half over, so N values take about N FP64 adds
-// instead of the 5 N of a tree per value (an FP64 instruction holds the pipe
-// for 16 cycles here).  Lane l ends with value l / (32 / N).
+// instead of the 5 N of a tree per value (an FP64 instruction of a warp holds its
+// SM quarter's pipe for 64 cycles here).  Lane l ends with value l / (32 / N).
 template <int N, int O>
 __device__ inline double warp_sums(const double (&v)[N]) {
   if constexpr (N == 1) {
@@ -2143,12 +2146,12 @@ __device__ inline void block_sums_out(const double* m, int content, double* part
 // thread, 115 in 7, 132 in 8).
 constexpr int MEAS_SPT = 8;
 __host__ __device__ inline int meas_spt(int V, bool f64) {
-  constexpr int W = 32 * 8 * 152;
+  constexpr int W = 32 * 8 * SMS;
   const int s = f64 && V > 2 * W ? (V + W - 1) / W : V / W;
   return s < 1 ? 1 : (s > MEAS_SPT ? MEAS_SPT : s);
 }
 // threads per block: one warp where blocks of BLOCK would leave SMs idle
-__host__ __device__ inline int meas_threads(int V) { return V <= 2 * 152 * BLOCK ? 32 : BLOCK; }
+__host__ __device__ inline int meas_threads(int V) { return V <= 2 * SMS * BLOCK ? 32 : BLOCK; }
 inline unsigned meas_blocks(int V, bool f64) {
   const int per = meas_spt(V, f64) * meas_threads(V);
   return (unsigned)((V + per - 1) / per);
@@ -2290,7 +2293,7 @@ __global__ void __launch_bounds__(BLOCK) k_flow(Fields<R> in, Fields<R> out, Geo
 // marker, most of that under the step's end (64^3, 20 steps: 581 us for the whole
 // flow, 606 with the step's blocks counting themselves in, 728 with a launch
 // before and one after each step).
-constexpr int FIXUP_BLOCKS = 152 * 8;
+constexpr int FIXUP_BLOCKS = 8 * SMS;
 template <typename R>
 __global__ void __launch_bounds__(256) k_flow_fixup(Fields<R> in, Fields<R> out, Geom g,
                                                     const unsigned long long* first_zero,

@@ -286,7 +286,7 @@ void append_segments(const su2gpu_pool* P, int s, int seg, std::vector<int4>& ou
 // 20^3 (3000) 301 against 286, 6 of 24^3 (1296) 207 against 250, 7 of 24^3 with
 // 21 smaller ones 1454 against 919.  FP64 warps on one quarter run one after
 // another, so FP64 teams have one warp per quarter in all (6 chains of 12^3 1006
-// against 1077 us, 24 of them, 648 warps, 3144 against 1489).
+// against 1077 us, 24 of them, 768 warps, 3144 against 1489).
 struct TeamShape { int blocks, threads, warps; };
 constexpr int TEAM_WARPS = 1600, TEAM_LARGE_WARPS = 1300, TEAM_WARPS_F64 = 608;
 bool team_shape(int prec, int half, TeamShape* t) {
@@ -334,8 +334,8 @@ int choose_teams(su2gpu_pool* P, bool fits) {
 // The groups of the automatic choice, for pools that neither the persistent nor
 // the team sweep takes: GROUP_STREAMS groups at a time on as many streams.
 // Passes of different groups then fill each other's launch gaps, ramps and
-// tails (one launch per pass issues instructions half of the time, four streams
-// three quarters), and where the pool exceeds L2, the chains in flight stay in
+// tails (one launch per pass issues in 52 % of the slots, the groups of the
+// 384-chain ensemble in 69 %), and where the pool exceeds L2, the chains in flight stay in
 // it from pass to pass: as many rounds as keep them to GROUP_BYTES, or one
 // round up to ONE_ROUND_BYTES.  Measured, us for the sweeps of a pool, one
 // launch per pass against this choice (the best of 50 group and stream counts):
