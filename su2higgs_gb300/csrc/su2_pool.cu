@@ -652,6 +652,17 @@ int enqueue_persist(su2gpu_pool* P, const int4* tiles, int nt, uint32_t* const* 
   return SU2GPU_OK;
 }
 
+// the pool's stream follows all of the streams that were forked from it
+int join_streams(su2gpu_pool* P, const std::vector<cudaStream_t>& ss) {
+  cudaError_t je = cudaSuccess;
+  for (size_t k = 0; k < ss.size(); k++) {
+    cudaError_t e = cudaEventRecord(P->grp_ev[k + 1], ss[k]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0);
+    if (e != cudaSuccess) je = e;
+  }
+  return je == cudaSuccess ? SU2GPU_OK : fail(SU2GPU_ERR_CUDA, "joining the update streams: %s", cudaGetErrorString(je));
+}
+
 // `nsweeps` sweeps of every chain by the teams: one launch per team shape, side
 // by side on the update streams when there are several, then the chains' sweep
 // counters + nsweeps (with sweeps)
@@ -674,16 +685,16 @@ int enqueue_teams(su2gpu_pool* P, uint32_t* const* sweeps, int nchains, int nswe
     PCK(cudaEventRecord(P->grp_ev[0], P->st));
     for (cudaStream_t st : ss) PCK(cudaStreamWaitEvent(st, P->grp_ev[0], 0));
   }
-  for (int k = 0; k < n; k++) {
+  cudaError_t le = cudaSuccess;
+  for (int k = 0; k < n && le == cudaSuccess; k++) {
     const su2gpu_pool::Team& t = P->teams[k];
     A.slots = (const int*)P->teamslots.p + t.first;
-    PCK(P->pers->team(P->nmuca > 0, t.blocks, t.threads, t.count, &A, ss[k % ss.size()]));
+    le = P->pers->team(P->nmuca > 0, t.blocks, t.threads, t.count, &A, ss[k % ss.size()]);
   }
+  if (le != cudaSuccess) cudaGetLastError();  // returned here, not by the next call
   if (n > 1)
-    for (int k = 0; k < (int)ss.size(); k++) {
-      PCK(cudaEventRecord(P->grp_ev[k + 1], ss[k]));
-      PCK(cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0));
-    }
+    if (int rc = join_streams(P, ss)) return rc;
+  if (le != cudaSuccess) return fail(SU2GPU_ERR_CUDA, "team sweep launch: %s", cudaGetErrorString(le));
   if (sweeps) launch_pool_next_sweep(sweeps, nchains, P->st, (uint32_t)nsweeps);
   PCK(cudaGetLastError());
   return SU2GPU_OK;
@@ -1270,14 +1281,8 @@ static int pool_enqueue(su2gpu_pool* P, int32_t nsweeps, int32_t use_graph) {
     };
     rc = fork();
     if (rc) cudaGetLastError();  // returned here, not by the next call
-    cudaError_t je = cudaSuccess;
-    for (int k = 0; k < NS; k++) {
-      cudaError_t e = cudaEventRecord(P->grp_ev[k + 1], ss[k]);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(P->st, P->grp_ev[k + 1], 0);
-      if (e != cudaSuccess) je = e;
-    }
-    if (rc) return rc;
-    if (je != cudaSuccess) return fail(SU2GPU_ERR_CUDA, "joining the groups' streams: %s", cudaGetErrorString(je));
+    const int jrc = join_streams(P, ss);
+    if (rc || jrc) return rc ? rc : jrc;
     std::vector<PassDesc> passes;
     sweep_recipe(P->recipe, passes, tot);
   } else if (use_graph) {

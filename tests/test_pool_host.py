@@ -188,3 +188,19 @@ def test_conversions_of_a_large_cycle_do_not_wait_behind_the_sweeps(env, monkeyp
     assert swept and len(moved) == 2  # upload and download streams
     assert (max(priority[a] for a in moved) <= min(priority[a] for a in swept)) == turns  # less is higher
     pool.close()
+
+
+@pytest.mark.parametrize("n", [0, 1, 2])
+def test_a_failing_team_leaves_no_stream_unjoined(env, n):
+    gpu, fake = env
+    pool = make_pool(gpu, [(4, 4, 4), (8, 8, 8), (8, 8, 16)])
+    assert pool.launches_per_sweep() == 3  # two shapes, and the sweep counters
+    fake.reset()
+    fake.fail("launch", n)
+    with pytest.raises(gpu.SU2GPUError):
+        pool.run(2)
+    worked, joined = forked_and_joined(fake.ops())
+    assert worked <= joined and len(joined) == 2
+    fake.reset()
+    pool.run(2)
+    pool.close()
