@@ -1558,6 +1558,16 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
   }
   std::vector<cudaEvent_t>& ev = P->cyc_ev;
   ConvItem* dit = (ConvItem*)P->d_items.p;
+  // a call that fails returns once nothing of it runs any more: its copies read
+  // and write the caller's arrays
+  std::vector<double> hs(sums ? (size_t)na * NSUMS : 0);
+  struct Drain {
+    std::vector<cudaStream_t> streams;
+    ~Drain() {
+      for (cudaStream_t st : streams) cudaStreamSynchronize(st);
+    }
+  } drain{ss};
+  drain.streams.insert(drain.streams.end(), {copy, down_copy, P->st});
   // the fields may still be in use by earlier work on st
   PCK(cudaEventRecord(ev[4 * G], P->st));
   PCK(cudaStreamWaitEvent(copy, ev[4 * G], 0));
@@ -1670,14 +1680,11 @@ int su2gpu_pool_cycle(su2gpu_pool* P, int32_t n, const int32_t* slots, const dou
     PCK(cudaEventRecord(ev[4 * G + 1 + k], ss[k]));
     PCK(cudaStreamWaitEvent(P->st, ev[4 * G + 1 + k], 0));
   }
-  std::vector<double> hs;
-  if (sums) {
-    hs.resize((size_t)na * NSUMS);
-    PCK(cudaMemcpyAsync(hs.data(), P->sums.p, hs.size() * 8, cudaMemcpyDeviceToHost, P->st));
-  }
+  if (sums) PCK(cudaMemcpyAsync(hs.data(), P->sums.p, hs.size() * 8, cudaMemcpyDeviceToHost, P->st));
   PCK(cudaStreamSynchronize(copy));
   PCK(cudaStreamSynchronize(down_copy));
   if ((rc = pool_check(P))) return rc;
+  drain.streams.clear();
   if (sums)
     for (int a = 0; a < na; a++) memcpy(sums + (size_t)pos[a] * NSUMS, hs.data() + (size_t)a * NSUMS, NSUMS * 8);
   for (int a = 0; a < na; a++) {

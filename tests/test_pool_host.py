@@ -204,3 +204,28 @@ def test_a_failing_team_leaves_no_stream_unjoined(env, n):
     fake.reset()
     pool.run(2)
     pool.close()
+
+
+@pytest.mark.parametrize("what,n", [("copy", 3), ("copy", 20), ("copy", 31), ("launch", 2), ("launch", 9), ("graph", 5),
+                                    ("wait", 12)])
+def test_a_failing_cycle_returns_with_nothing_in_flight(env, monkeypatch, what, n):
+    # its copies read and write the caller's arrays
+    gpu, fake = env
+    monkeypatch.setenv("SU2GPU_CYCLE_GROUPS", "4")
+    sides = [(4, 6, 8)] * 8
+    pool = make_pool(gpu, sides)
+    fields = [{"link": np.zeros((192, 3, 4)), "trip": np.zeros((192, 3))} for _ in sides]
+    pool.cycle(list(pool.active()), fields, 2)  # graphs, rings and tables are made
+    fake.reset()
+    fake.fail(what, n)
+    with pytest.raises(gpu.SU2GPUError):
+        pool.cycle(list(pool.active()), fields, 2)
+    assert fake.failed(what)
+    busy = set()
+    for w, a, _ in fake.ops():
+        if w in ("copy", "fill", "launch", "graph"):
+            busy.add(a)
+        if w == "sync":
+            busy.discard(a)
+    assert not busy
+    pool.close()
