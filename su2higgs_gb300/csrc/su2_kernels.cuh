@@ -637,7 +637,7 @@ __device__ inline int overrelax_f64(double (&p)[N], const double (&s)[N], double
     Ysq += y[k] * y[k];
   }
   // (V(x) - V(X)) / (x - X) = C x^3 + b x^2 + c x + d
-  const double b = C * X, c = fma(b, X, B + 2.0 * Ysq * C);
+  const double b = C * X, c = B + C * fma(X, X, 2.0 * Ysq);
   const double newX = polysolve3<double>(C, b, c, fma(c, X, F), fallback);
   const double dV = fma(fma(4.0 * C, fma(X, X, Ysq), 2.0 * B), X, F);
   const double dVn = fma(fma(4.0 * C, fma(newX, newX, Ysq), 2.0 * B), newX, F);
