@@ -611,7 +611,7 @@ __device__ inline int metro_doublet_f64(const Fields<double>& f, const CoupT<dou
 // |v| and v / |v| from v^2: CUDA's reciprocal root, and from it by one Newton step
 // each the root and the direction, as exact as with sqrt and a division per
 // component.  (|v| as v^2 rsqrt(v^2), and a direction by one reciprocal, cost the
-// overrelaxation 12 % in rms error: 1.45 against 1.30 units of 2^-53; with these 1.25.)
+// overrelaxation 12 % in rms error: 1.45 against 1.30 units of 2^-53; with these 1.20.)
 template <int N>
 __device__ inline double direction_f64(const double (&v)[N], double vsq, double (&e)[N]) {
   const double y = rsqrt(vsq), r = vsq * y, F = fma(0.5 * y, fma(-r, r, vsq), r), dy = y * fma(-F, y, 1.0);
@@ -2102,21 +2102,29 @@ __device__ inline double warp_sums(const double (&v)[N]) {
 }
 
 // sums of m[] over the block (blockDim.x a multiple of 32, at most BLOCK) to
-// partials[k * nblocks + block].  The runtime content sums all NSUMS values
-// (those that its fields do not have are 0 and are left out below): one tree per
-// value that it has takes longer from seven values on.
+// partials[k * nblocks + block].  The runtime content sums the first 16 values,
+// and the others if its fields have any of them (a value that they do not have is
+// left out below): one tree per value that it has takes longer from six on.
 template <int CC>
 __device__ inline void block_sums_out(const double* m, int content, double* partials, int nblocks, int block) {
   constexpr int NA = nactive_sums<CC>();
-  constexpr int N = CC == C_GENERIC ? 32 : (NA <= 4 ? 4 : (NA <= 8 ? 8 : (NA <= 16 ? 16 : 32)));
+  constexpr int N = CC == C_GENERIC ? NSUMS : (NA <= 4 ? 4 : (NA <= 8 ? 8 : (NA <= 16 ? 16 : 32)));
   __shared__ double sm[BLOCK / 32][N];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int j = -1;  // this thread's sum: its place in sm[w]
   if constexpr (CC == C_GENERIC) {
-    double v[N];
+    double v[16], u[8];
 #pragma unroll
-    for (int q = 0; q < N; q++) v[q] = q < NSUMS ? m[q < NSUMS ? q : 0] : 0.0;
-    sm[w][lane] = warp_sums<N, 16>(v);
+    for (int q = 0; q < 16; q++) v[q] = m[q];
+    const double r = warp_sums<16, 16>(v);
+    if (!(lane & 1)) sm[w][lane / 2] = r;
+    static_assert(NSUMS == 24, "16 and 8 sums");
+    if (content & (C_T | C_S)) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) u[q] = m[16 + q];
+      const double t = warp_sums<8, 16>(u);
+      if (!(lane & 3)) sm[w][16 + lane / 4] = t;
+    }
     if (threadIdx.x < NSUMS && sum_active(threadIdx.x, content)) j = threadIdx.x;
   } else {
     double v[N];

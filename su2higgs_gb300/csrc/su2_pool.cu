@@ -491,7 +491,7 @@ int rebuild(su2gpu_pool* P, void* arena_base = nullptr, void* slot_base = nullpt
     sp.clear();
     for (int s : P->active) {
       first.push_back((int)mt.size());
-      const int V = P->slots[s].g.V, spt = pool_meas_spt(V, P->prec == 64, P->ops->content == C_GENERIC);
+      const int V = P->slots[s].g.V, spt = pool_meas_spt(V);
       for (int t0 = 0; t0 < V; t0 += BLOCK * spt) mt.push_back(int2{s, t0});
       sp.push_back((uint32_t*)(sb + (size_t)s * 256));
     }

@@ -538,11 +538,9 @@ __global__ void k_pool_next_sweep(uint32_t* const* sweeps, int n, uint32_t inc) 
 #endif
 
 // Sites per thread of a pool chain's measurement: a pool has other chains to
-// fill the SMs, so only small chains are cut finer than MEAS_SPT (the smallest of
-// an FP32 pool of the runtime content less so: its blocks' sums weigh more).  A
-// function of the chain and the pool's kind alone, as the sums depend on it.
-__host__ __device__ inline int pool_meas_spt(int V, bool f64, bool generic) {
-  return V <= 8192 ? (generic && !f64 ? 2 : 1) : (V <= 32768 ? 2 : MEAS_SPT);
+// fill the SMs, so only small chains are cut finer than MEAS_SPT.
+__host__ __device__ inline int pool_meas_spt(int V) {
+  return V <= 8192 ? 1 : (V <= 32768 ? 2 : MEAS_SPT);
 }
 
 // measurement over every chain: tiles of pool_meas_spt sites per thread of
@@ -550,7 +548,7 @@ __host__ __device__ inline int pool_meas_spt(int V, bool f64, bool generic) {
 // reduced per chain.  The magnetic charge's projections are computed where
 // they are needed (no per-chain scratch planes).
 template <typename R, int CC>
-__global__ void __launch_bounds__(BLOCK, CC == C_GENERIC && sizeof(R) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(BLOCK, CC == C_GENERIC && sizeof(R) == 4 ? 4 : 0)
     k_pool_measure(PoolArgs a, double* partials) {
   int2 tile = a.tiles[blockIdx.x];
   if (bad_tile(a, tile)) return;
@@ -558,7 +556,7 @@ __global__ void __launch_bounds__(BLOCK, CC == C_GENERIC && sizeof(R) == 4 ? 4 :
   double m[NSUMS];
 #pragma unroll
   for (int k = 0; k < NSUMS; k++) m[k] = 0.0;
-  const int spt = pool_meas_spt(d.g.V, sizeof(R) == 8, CC == C_GENERIC);
+  const int spt = pool_meas_spt(d.g.V);
   for (int j = 0; j < spt; j++) {
     int t = tile.y + j * BLOCK + threadIdx.x;
     if (t < d.g.V) measure_site<R, CC>(d.f, d.g, d.cp, t, AlphaOnTheFly{}, m);
