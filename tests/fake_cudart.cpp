@@ -1,7 +1,7 @@
 // fake_cudart.cpp -- a CUDA runtime without a GPU, for tests of the library's
 // host code: device memory is host memory, copies and fills are done at once,
 // kernels are not run.  What the host code asks for is written to a log, and a
-// test can make the n-th call of a function fail or choose what events measure.
+// test can make the n-th call of a function fail.
 // Linked with the library's own objects instead of the CUDA runtime.
 #include <cuda_runtime_api.h>
 
@@ -9,7 +9,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
-#include <set>
 #include <string>
 #include <vector>
 
@@ -23,9 +22,7 @@ std::map<std::string, int> fail_after;  // function -> successful calls before t
 std::map<void*, size_t> blocks;
 int64_t live = 0;
 cudaError_t last = cudaSuccess;
-std::set<cudaStream_t> capturing;
 int64_t numbers = 0;
-float elapsed = 1.0f;
 std::map<const void*, std::string> names;  // kernels by the address of their host stub
 std::string watched;
 int watched_arg = 0;
@@ -56,10 +53,9 @@ cudaError_t step(const char* what, const void* a, const void* b) {
 
 extern "C" {
 // ---- the test's side
-void fake_reset() { ops.clear(); fail_after.clear(); elapsed = 1.0f; last = cudaSuccess; watched.clear(); }
+void fake_reset() { ops.clear(); fail_after.clear(); last = cudaSuccess; watched.clear(); }
 void fake_fail(const char* what, int n) { fail_after[what] = n; }
 int fake_failed(const char* what) { return !fail_after.count(what); }
-void fake_elapsed(float ms) { elapsed = ms; }
 int64_t fake_live_bytes() { return live; }
 // the 8 bytes of argument `arg` of the kernel whose name holds `name`, at its last launch
 void fake_watch(const char* name, int arg) { watched = name; watched_arg = arg; watched_value = 0; }
@@ -165,14 +161,11 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t st) { return step("record", st, e); }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = elapsed; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t st, cudaStreamCaptureMode) {
-  if (cudaError_t e = step("begin capture", st)) return e;
-  capturing.insert(st);
-  return cudaSuccess;
+  return step("begin capture", st);
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t st, cudaGraph_t* g) {
-  capturing.erase(st);
   *g = nullptr;
   if (cudaError_t e = step("end capture", st)) return e;
   *g = (cudaGraph_t)handle();

@@ -27,7 +27,6 @@ class Fake:
         self.lib = lib
         lib.fake_op.restype = ctypes.c_char_p
         lib.fake_live_bytes.restype = ctypes.c_int64
-        lib.fake_elapsed.argtypes = [ctypes.c_float]
         lib.fake_watched.restype = ctypes.c_uint64
         lib.fake_room.restype = ctypes.c_int64
         lib.fake_room.argtypes = [ctypes.c_uint64]
